@@ -87,6 +87,7 @@ void launch_bwd_diag(const DevStruct &, const int *, int, int, const T *, int, T
 template <typename T>
 void launch_diag_scale(const DevStruct &, int, const T *, T *, int, int, cudaStream_t);
 int solve_rows_per_tile();
+cudaError_t set_solve_attrs();
 // vec.cu
 void spmv_partition(int n, const int *rowptr, std::vector<int> &part);
 void launch_spmv_stream(int nblocks, const int *part, const int *rowptr, const int *col, const double *val,
@@ -1475,12 +1476,21 @@ static int device_setup(pastix_data_t *pd) {
         CUDA_TRY((pgpu::set_smem_attrs<float, pgpu::FACT_POTRF>(mx, mx, mx)));
         CUDA_TRY((pgpu::set_smem_attrs<float, pgpu::FACT_SYTRF>(mx, mx, mx)));
         CUDA_TRY((pgpu::set_smem_attrs<float, pgpu::FACT_GETRF>(mx, mx, mx)));
+        CUDA_TRY(pgpu::set_solve_attrs());
         attrs = true;
     }
     CUDA_TRY(cudaStreamSynchronize(st));
     d.ready = true;
     return PASTIX_SUCCESS;
 }
+
+// Programmatic dependent launches (launch_k) on this host thread for a scope.
+namespace {
+struct PdlScope {
+    explicit PdlScope(bool on) { pgpu::set_pdl(on); }
+    ~PdlScope() { pgpu::set_pdl(false); }
+};
+}  // namespace
 
 // ---------------------------------------------------------------------------
 // numerical factorization
@@ -1501,10 +1511,7 @@ static int run_factor(pastix_data_t *pd, double criterion) {
     const cudaStream_t sd = two ? d.side : st;
     // FP32 (launched kernel by kernel, not as a graph): each launch of the level
     // chain overlaps the end of the kernel ahead of it (programmatic dependent launch)
-    struct PdlScope {
-        explicit PdlScope(bool on) { pgpu::set_pdl(on); }
-        ~PdlScope() { pgpu::set_pdl(false); }
-    } pdl_scope(two);
+    PdlScope pdl_scope(two);
     if constexpr (sizeof(T) == 4)
         CUDA_TRY(cudaMemsetAsync(d.queues.p, 0, 3 * pd->levels.size() * sizeof(int), st));
     if (two) {
@@ -1888,6 +1895,9 @@ static void solve_perm(pastix_data_t *pd, int trans, T *Y, int ldy, int nrhs) {
     const T *L = reinterpret_cast<const T *>(d.Lc.p);
     const T *U = reinterpret_cast<const T *>(d.Uc.p);
     int fk = fact_kind(pd);
+    // each kernel of the sweeps loads its part of the factor while the one ahead
+    // finishes (with per-launch timing events in between there is nothing to overlap)
+    PdlScope pdl_scope(!pd->prof_on);
     if (fk == pgpu::FACT_POTRF) {
         sweep_forward<T>(pd, L, 0, 0, 0, Y, ldy, nrhs);
         sweep_backward<T>(pd, L, 0, 0, 0, Y, ldy, nrhs);

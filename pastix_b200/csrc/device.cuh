@@ -82,7 +82,14 @@ struct DevStruct {
 // Without such a launch it returns at once.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launches of the FP32 factorization's level chains may overlap the launch of
+// Lets the next kernel of the stream be scheduled as soon as every block of this
+// one has called it (or ended) instead of when this one ends: that kernel loads
+// what does not depend on this one and then waits in pdl_wait.  A kernel that
+// is scheduled ahead never holds up the earlier ones, whose blocks are all
+// resident by then.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launches of the FP32 factorization's level chains and of the solve sweeps may overlap the launch of
 // each kernel with the end of the one ahead of it in its stream (every kernel
 // launched this way waits in pdl_wait first); switched on per host thread by
 // set_pdl.
@@ -114,6 +121,29 @@ struct FactParams {
     int *status;                // device status word (0 = fine)
     double *dscr;               // k_diag_cluster: the finished panels of each cblk of a launch, DC_SCR_DOUBLES per cblk
 };
+
+// Asynchronous copies of one element global -> shared (zero when !valid), and
+// the FP64 tensor core product D (8 x 8) += A (8 x 4) B (4 x 8): lane 4 g + t
+// holds A(g, t), B(t, g), D(g, 2 t) and D(g, 2 t + 1).
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid) {
+    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    int sz = valid ? 8 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+__device__ __forceinline__ void dmma884(double &d0, double &d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem, bool valid) {
+    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    int sz = valid ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
+}
 
 // Element-wise transfer by a whole CTA with UNR independent loads in flight per
 // thread: st(e, ld(e)) for e in [0, total).  All loads of a batch are issued

@@ -744,21 +744,6 @@ constexpr int DM_BM = 128, DM_BN = 64, DM_BK = 16;
 constexpr int DM_LDA = DM_BM + 8, DM_LDB = DM_BN + 8;  // row strides = 8 mod 16 doubles: 2 wavefronts per fragment load
 constexpr size_t DM_SMEM = sizeof(double) * 2 * DM_BK * (DM_LDA + DM_LDB);
 
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid) {
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    int sz = valid ? 8 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
-__device__ __forceinline__ void dmma884(double &d0, double &d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 template <int FACT>
 __global__ void __launch_bounds__(256) k_update_dmma(DevStruct s, const UpdTile *__restrict__ tiles, double *L,
                                                       double *U) {
@@ -2321,12 +2306,6 @@ constexpr int TI_ZLD = 36;  // row stride of Z_i (floats): conflict-free fragmen
 __host__ __device__ inline int ti_ts_ld(int maxnzb) { return 32 * maxnzb + 4; }
 __host__ __device__ inline long long trinv_smem_bytes(int maxnzb) {
     return 32LL * maxnzb * DG_LD * 8 + 2 * 32LL * (ti_ts_ld(maxnzb) + TI_ZLD) * 4;
-}
-
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem, bool valid) {
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    int sz = valid ? 4 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
 }
 
 // T^{-1} of the diagonal block of a cblk, one 32-column block column j per
