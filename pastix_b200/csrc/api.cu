@@ -86,6 +86,17 @@ template <typename T>
 void launch_bwd_diag(const DevStruct &, const int *, int, int, const T *, int, T *, int, int, cudaStream_t);
 template <typename T>
 void launch_diag_scale(const DevStruct &, int, const T *, T *, int, int, cudaStream_t);
+// update_i8.cu
+long long i8_image_bytes(int, int);
+int i8_max_k();
+void launch_split_i8(const DevStruct &, const SplitSlab *, int, const double *, const double *, const int64_t *,
+                     unsigned char *, double *, int, cudaStream_t);
+template <int F>
+void launch_update_i8(const DevStruct &, const UpdTile *, int, double *, double *, const unsigned char *,
+                      const unsigned char *, const double *, const double *, const int64_t *, int *, int *, int,
+                      cudaStream_t);
+cudaError_t set_i8_attrs();
+int sm_count();
 int solve_rows_per_tile();
 cudaError_t set_solve_attrs();
 // vec.cu
@@ -135,6 +146,10 @@ enum : int {
 
 namespace {
 
+// FP64 update tasks with a source this wide and a blok this tall take the
+// integer-slice tiles, the others DMMA or FMA tiles: a K block is 32 columns and
+// the least N of a tile 16, so that below these lines most of a product is padding.
+constexpr idx_t I8_MIN_K = 32, I8_MIN_N = 8;
 constexpr idx_t SMALL_PANEL_ELEMS = 4096;  // st*nc below which a cblk is factored in one CTA's smem
 
 template <typename X>
@@ -171,6 +186,9 @@ struct LevelLists {
     int upds0, upds1;       // k_update tiles (64 x 64), FP32 factors (tasks the tcgen05 kernel does not take)
     int updb0, updb1;       // big update tiles (128 x 64): DMMA for FP64
     int updt0, updt1;       // the same tasks in 128-row aligned windows: tcgen05 for FP32
+    int updm, updbm;        // FP64 lists: tiles from here on belong to tasks that the integer kernel takes
+    int upi0, upi1;         // those tasks in 128 x 128 windows: integer slices on tcgen05 (FP64 factors)
+    int isl0, isl1;         // 128-row slabs of their source cblks, cut into digits
     int updtn, updsn;       // FP32 lists: tiles before these target the next level's cblks
     int spl0, spl1;         // 128-row slabs of the level's cblks split into BF16 terms (FP32)
     int tt0, tt1;           // FP32 TRSM as GEMM tiles (tcgen05), task = cblk
@@ -207,7 +225,13 @@ struct Device {
     DBuf<pgpu::TaskDev> tasks;
     DBuf<int> small_list, large_list, level_cblks;
     DBuf<pgpu::RowTile> trsm_tiles, solve_tiles;
-    DBuf<pgpu::UpdTile> upd_tiles, upd_big_tiles, upd_tc_tiles, upd_tiles32;
+    DBuf<pgpu::UpdTile> upd_tiles, upd_big_tiles, upd_tc_tiles, upd_tiles32, upd_i8_tiles;
+    // FP64: digit images of the level's source panels (L and, per kind, L D or U), their row scales
+    DBuf<pgpu::SplitSlab> i8_slabs;
+    DBuf<int64_t> i8_off;
+    DBuf<unsigned char> i8_img0, i8_img1;
+    DBuf<double> i8_sc0, i8_sc1;
+    bool i8_on = false;      // the images of this factorization fit the device
     // matrix
     DBuf<double> vals, csr_val;
     DBuf<int64_t> lmap, umap, csr_src, perm;
@@ -282,7 +306,10 @@ struct pastix_data_s {
     // host copies of the launch lists
     std::vector<int> small_list, large_list, level_cblks;
     std::vector<pgpu::RowTile> trsm_tiles, solve_tiles;
-    std::vector<pgpu::UpdTile> upd_tiles, upd_big_tiles, upd_tc_tiles, upd_tiles32;
+    std::vector<pgpu::UpdTile> upd_tiles, upd_big_tiles, upd_tc_tiles, upd_tiles32, upd_i8_tiles;
+    std::vector<pgpu::SplitSlab> i8_slabs;
+    std::vector<int64_t> i8_off;             // byte offset of each cblk's digit image in its level's images (-1: none)
+    int64_t i8_total = 0;                    // bytes of the largest level's images
     std::vector<pgpu::TaskDev> tasks;
     std::vector<int64_t> cb_dinv;
     std::vector<int64_t> sp_off;             // byte offset of each cblk's BF16 image (-1: none)
@@ -1097,6 +1124,10 @@ static int build_maps_and_lists(pastix_data_t *pd) {
     pd->trsm_tiles.clear(); pd->solve_tiles.clear(); pd->upd_tiles.clear(); pd->upd_big_tiles.clear();
     pd->upd_tc_tiles.clear();
     pd->upd_tiles32.clear();
+    pd->upd_i8_tiles.clear();
+    pd->i8_slabs.clear();
+    pd->i8_off.assign(sv.cblknbr, -1);
+    pd->i8_total = 0;
     // exclusive tasks: dst targeted by a single source in the level
     pd->tasks.resize(sv.tasks.size());
     {
@@ -1237,24 +1268,70 @@ static int build_maps_and_lists(pastix_data_t *pd) {
         L.updt0 = (int)pd->upd_tc_tiles.size();
         L.upds0 = (int)pd->upd_tiles32.size();
         std::vector<pgpu::UpdTile> tc_far, s32_far;  // tiles whose target is two or more levels up
+        L.upi0 = (int)pd->upd_i8_tiles.size();
+        L.isl0 = (int)pd->i8_slabs.size();
+        // FP64 tasks of the integer kernel: their DMMA / FMA tiles go to the end of the
+        // lists, where a factorization whose images do not fit the device finds them
+        auto i8_task = [&](const pgpu::Task &tk) {
+            const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
+            return K >= I8_MIN_K && K <= pgpu::i8_max_k() && tk.n >= I8_MIN_N;
+        };
+        for (int part = 0; part < 2; part++) {
+            if (part) {
+                L.updm = (int)pd->upd_tiles.size();
+                L.updbm = (int)pd->upd_big_tiles.size();
+            }
+            for (idx_t t = sv.lvl_task_ptr[l]; t < sv.lvl_task_ptr[l + 1]; t++) {
+                const auto &tk = sv.tasks[t];
+                const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
+                if (K * sv.cb_stride[tk.src] <= SMALL_PANEL_ELEMS) continue;  // done by k_panel_small
+                const bool i8 = i8_task(tk);
+                if (i8 != (part == 1)) continue;
+                const bool big = tk.n >= pd->tune_dmma_n && K >= pd->tune_dmma_k;  // DMMA tiles
+                const idx_t BM = big ? 128 : 64, BN = 64;
+                auto &list = big ? pd->upd_big_tiles : pd->upd_tiles;
+                for (int side = 0; side < (fk == pgpu::FACT_GETRF ? 2 : 1); side++) {
+                    const idx_t M = tk.m - (side ? tk.n : 0);
+                    if (M <= 0) continue;
+                    const idx_t mt = (M + BM - 1) / BM, ntl = (tk.n + BN - 1) / BN;
+                    for (idx_t a = 0; a < mt; a++)
+                        for (idx_t c = 0; c < ntl; c++) {
+                            // symmetric kinds: skip tiles strictly above the diagonal of the square part
+                            if (fk != pgpu::FACT_GETRF && (a + 1) * BM <= c * BN) continue;
+                            list.push_back(pgpu::UpdTile{(int)t, (int)a, (int)c, side});
+                        }
+                    if (!i8) continue;
+                    const idx_t ra = tk.row0 + (side ? tk.n : 0);
+                    const idx_t mi = (ra % 8 + M + 127) / 128, ni = (tk.row0 % 8 + tk.n + 127) / 128;
+                    for (idx_t a = 0; a < mi; a++)
+                        for (idx_t c = 0; c < ni; c++)
+                            if (fk == pgpu::FACT_GETRF || (a + 1) * 128 > c * 128)
+                                pd->upd_i8_tiles.push_back(pgpu::UpdTile{(int)t, (int)a, (int)c, side});
+                }
+                if (i8) pd->i8_off[tk.src] = 0;
+            }
+        }
+        {  // the images of a level's sources; the next level overwrites them
+            int64_t bytes = 0;
+            for (idx_t p = sv.lvl_ptr[l]; p < sv.lvl_ptr[l + 1]; p++) {
+                const idx_t k = sv.lvl_cblk[p];
+                if (pd->i8_off[k] < 0) continue;
+                pd->i8_off[k] = bytes;
+                bytes += pgpu::i8_image_bytes((int)(sv.cb_lcol[k] - sv.cb_fcol[k] + 1), (int)sv.cb_stride[k]);
+                for (idx_t r = 0; r < sv.cb_stride[k]; r += 128) pd->i8_slabs.push_back(pgpu::SplitSlab{(int)k, (int)r});
+            }
+            pd->i8_total = std::max(pd->i8_total, bytes);
+        }
+        L.upi1 = (int)pd->upd_i8_tiles.size();
+        L.isl1 = (int)pd->i8_slabs.size();
         for (idx_t t = sv.lvl_task_ptr[l]; t < sv.lvl_task_ptr[l + 1]; t++) {
             const auto &tk = sv.tasks[t];
             const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
             if (K * sv.cb_stride[tk.src] <= SMALL_PANEL_ELEMS) continue;  // done by k_panel_small
-            const bool big = tk.n >= pd->tune_dmma_n && K >= pd->tune_dmma_k;  // FP64: DMMA tiles
             const bool tc = K >= pd->tune_tc_k;                                // FP32: tcgen05 tiles
-            const idx_t BM = big ? 128 : 64, BN = 64;
-            auto &list = big ? pd->upd_big_tiles : pd->upd_tiles;
             for (int side = 0; side < (fk == pgpu::FACT_GETRF ? 2 : 1); side++) {
                 idx_t M = tk.m - (side ? tk.n : 0);
                 if (M <= 0) continue;
-                idx_t mt = (M + BM - 1) / BM, ntl = (tk.n + BN - 1) / BN;
-                for (idx_t a = 0; a < mt; a++)
-                    for (idx_t c = 0; c < ntl; c++) {
-                        // symmetric kinds: skip tiles strictly above the diagonal of the square part
-                        if (fk != pgpu::FACT_GETRF && (a + 1) * BM <= c * BN) continue;
-                        list.push_back(pgpu::UpdTile{(int)t, (int)a, (int)c, side});
-                    }
                 const bool near = sv.cb_level[tk.dst] == (idx_t)l + 1;
                 if (!tc) {  // FP32 tasks with a narrow source: SIMT 64 x 64 tiles
                     const idx_t mt3 = (M + 63) / 64, nt3 = (tk.n + 63) / 64;
@@ -1427,6 +1504,9 @@ static int device_setup(pastix_data_t *pd) {
     CUDA_TRY(d.upd_big_tiles.upload(pd->upd_big_tiles, st));
     CUDA_TRY(d.upd_tc_tiles.upload(pd->upd_tc_tiles, st));
     CUDA_TRY(d.upd_tiles32.upload(pd->upd_tiles32, st));
+    CUDA_TRY(d.upd_i8_tiles.upload(pd->upd_i8_tiles, st));
+    CUDA_TRY(d.i8_slabs.upload(pd->i8_slabs, st));
+    CUDA_TRY(d.i8_off.upload(pd->i8_off, st));
     CUDA_TRY(d.sp_off.upload(pd->sp_off, st));
     CUDA_TRY(d.ti_off.upload(pd->ti_off, st));
     CUDA_TRY(d.ti_img.upload(pd->ti_img, st));
@@ -1477,6 +1557,7 @@ static int device_setup(pastix_data_t *pd) {
         CUDA_TRY((pgpu::set_smem_attrs<float, pgpu::FACT_SYTRF>(mx, mx, mx)));
         CUDA_TRY((pgpu::set_smem_attrs<float, pgpu::FACT_GETRF>(mx, mx, mx)));
         CUDA_TRY(pgpu::set_solve_attrs());
+        CUDA_TRY(pgpu::set_i8_attrs());
         attrs = true;
     }
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -1512,7 +1593,7 @@ static int run_factor(pastix_data_t *pd, double criterion) {
     // FP32 (launched kernel by kernel, not as a graph): each launch of the level
     // chain overlaps the end of the kernel ahead of it (programmatic dependent launch)
     PdlScope pdl_scope(two);
-    if constexpr (sizeof(T) == 4)
+    if (sizeof(T) == 4 || d.i8_on)
         CUDA_TRY(cudaMemsetAsync(d.queues.p, 0, 3 * pd->levels.size() * sizeof(int), st));
     if (two) {
         CUDA_TRY(cudaEventRecord(d.ev_chain[0], st));
@@ -1555,8 +1636,9 @@ static int run_factor(pastix_data_t *pd, double criterion) {
             });
         }
         if constexpr (sizeof(T) == 8) {
-            launch_cls(pd, PC_UPDATE, lv.upd1 - lv.upd0, [&] {
-                pgpu::launch_update<T, F>(d.ds, d.upd_tiles.p + lv.upd0, lv.upd1 - lv.upd0, L, U, st);
+            const int n = (d.i8_on ? lv.updm : lv.upd1) - lv.upd0;
+            launch_cls(pd, PC_UPDATE, n, [&] {
+                pgpu::launch_update<T, F>(d.ds, d.upd_tiles.p + lv.upd0, n, L, U, st);
             });
         } else {
             launch_cls(pd, PC_UPDATE, lv.updsn - lv.upds0, [&] {
@@ -1596,9 +1678,27 @@ static int run_factor(pastix_data_t *pd, double criterion) {
                 sd);
             if (two) CUDA_TRY(cudaEventRecord(d.ev_rest[l], d.side));
         } else {
-            launch_cls(pd, PC_UPDATE_BIG, lv.updb1 - lv.updb0, [&] {
-                pgpu::launch_update_big<T, F>(d.ds, d.upd_big_tiles.p + lv.updb0, lv.updb1 - lv.updb0, L, U, st);
+            const int n = (d.i8_on ? lv.updbm : lv.updb1) - lv.updb0;
+            launch_cls(pd, PC_UPDATE_BIG, n, [&] {
+                pgpu::launch_update_big<T, F>(d.ds, d.upd_big_tiles.p + lv.updb0, n, L, U, st);
             });
+            if (d.i8_on) {
+                const int nsl = lv.isl1 - lv.isl0;
+                launch_cls(pd, PC_SPLIT, nsl, [&] {
+                    const pgpu::SplitSlab *sl = d.i8_slabs.p + lv.isl0;
+                    pgpu::launch_split_i8(d.ds, sl, nsl, L, L, d.i8_off.p, d.i8_img0.p, d.i8_sc0.p,
+                                          F == pgpu::FACT_POTRF ? 0 : 1, st);
+                    if (F == pgpu::FACT_SYTRF)
+                        pgpu::launch_split_i8(d.ds, sl, nsl, L, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 2, st);
+                    if (F == pgpu::FACT_GETRF)
+                        pgpu::launch_split_i8(d.ds, sl, nsl, U, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 3, st);
+                });
+                launch_cls(pd, PC_UPDATE_BIG, lv.upi1 - lv.upi0, [&] {
+                    pgpu::launch_update_i8<F>(d.ds, d.upd_i8_tiles.p + lv.upi0, lv.upi1 - lv.upi0, L, U, d.i8_img0.p,
+                                              d.i8_img1.p, d.i8_sc0.p, d.i8_sc1.p, d.i8_off.p, d.queues.p + 3 * l,
+                                              d.counters.p + 1, pgpu::sm_count(), st);
+                });
+            }
         }
     }
     if (two) {  // the library stream resumes once every far update is in
@@ -1721,6 +1821,23 @@ extern "C" int pastix_subtask_bcsc2ctab(pastix_data_t *pd) {
         d.tinv.reset();
         d.timg.reset();
     }
+    // FP64: digit images of one level's panels; a factorization for which they do not fit runs on DMMA
+    d.i8_on = false;
+    if (!pd->mixed && pd->i8_total > 0) {
+        const size_t ib = (size_t)pd->i8_total, nr = pd->solver.rowidx.size();
+        const bool two = fk != pgpu::FACT_POTRF;
+        d.i8_on = d.i8_img0.alloc(ib) == cudaSuccess && d.i8_sc0.alloc(nr) == cudaSuccess &&
+                  (!two || (d.i8_img1.alloc(ib) == cudaSuccess && d.i8_sc1.alloc(nr) == cudaSuccess));
+        if (!d.i8_on) (void)cudaGetLastError();
+    }
+    if (!d.i8_on || fk == pgpu::FACT_POTRF) {
+        d.i8_img1.reset();
+        d.i8_sc1.reset();
+    }
+    if (!d.i8_on) {
+        d.i8_img0.reset();
+        d.i8_sc0.reset();
+    }
     CUDA_TRY(cudaMemsetAsync(d.Lc.p, 0, bytes, d.stream));
     if (d.Uc.p) CUDA_TRY(cudaMemsetAsync(d.Uc.p, 0, bytes, d.stream));
     const int64_t *um = d.Uc.p ? d.umap.p : nullptr;
@@ -1765,7 +1882,9 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
         else rc = run_factor<float, pgpu::FACT_GETRF>(pd, threshold);
     } else {
         // FP64: the whole level sequence is one CUDA graph per (kind, buffers)
-        const std::vector<uintptr_t> key{1, (uintptr_t)fk, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p};
+        const std::vector<uintptr_t> key{1, (uintptr_t)fk, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p,
+                                         (uintptr_t)d.i8_img0.p, (uintptr_t)d.i8_img1.p, (uintptr_t)d.i8_sc0.p,
+                                         (uintptr_t)d.i8_sc1.p};
         rc = run_graphed(pd, key, [&]() -> int {
             if (fk == pgpu::FACT_POTRF) return run_factor<double, pgpu::FACT_POTRF>(pd, threshold);
             if (fk == pgpu::FACT_SYTRF) return run_factor<double, pgpu::FACT_SYTRF>(pd, threshold);

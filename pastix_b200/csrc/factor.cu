@@ -20,6 +20,7 @@
 // the criterion is replaced by the criterion (POTRF) or by +/- criterion
 // keeping its sign (GETRF, SYTRF), and counted.
 #include "device.cuh"
+#include "tcgen05.cuh"
 
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -1093,7 +1094,6 @@ __device__ __forceinline__ void dg_pivot(double a, double crit, int &np, double 
 
 constexpr int DG_BLD = 34;        // row stride (doubles) of the published factor steps
 constexpr int DG_SPIN = 1 << 22;  // bound on a warp's wait for the factorization's progress
-constexpr int PGPU_STATUS_TIMEOUT = 3;
 
 // One warp: factor the nb x nb top block held row major in W (ld DG_LD) in
 // place, one row per lane in registers, with static pivoting; returns the
@@ -2143,15 +2143,12 @@ constexpr int TC_CH = TC_BK / 8;                    // 8-column chunks per K blo
 constexpr int TC_GROUP = 128 * TC_CH;               // bytes of 8 rows x TC_BK columns of one term
 constexpr int TC_PIECE = (TC_BM / 8) * TC_GROUP;    // one term of a 128-row operand block
 constexpr int TC_STAGE = 6 * TC_PIECE;              // A0 A1 A2 B0 B1 B2
-constexpr int TC_SPIN = 1 << 20;                    // try_wait rounds before giving up
 
 __host__ __device__ inline int split_nkb(int nc) { return (nc + TC_BK - 1) / TC_BK; }
 __host__ __device__ inline int split_ng(int st) { return (st + 7) / 8 + 16; }
 __host__ __device__ inline long long split_bytes(int nc, int st) {
     return 3LL * split_nkb(nc) * split_ng(st) * TC_GROUP;
 }
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Shared memory matrix descriptor: K-major, no swizzle; the next 8 K elements
 // 128 bytes on (LBO), the next 8 rows TC_GROUP bytes on (SBO); version 1.
@@ -2168,40 +2165,6 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t ad, uint64_t bd, 
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
         "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
-}
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-// Bounded wait for the completion of the phase of `bar` with parity `parity`.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-    const uint32_t a = smem_u32(bar);
-    for (int it = 0; it < TC_SPIN; it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// Bulk copy global -> shared (this GPU's memory, no multicast), completion on `bar`.
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
     uint32_t r[16];
@@ -2498,9 +2461,6 @@ constexpr int TP_STAGES = 2;
 constexpr size_t TP_SMEM = (size_t)TP_STAGES * TC_STAGE;
 constexpr int TP_THREADS = 192;
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // OR of `pred` over the 128 epilogue threads (named barrier 1, which also orders them)
 __device__ __forceinline__ int epi_bar_or(int pred) {
     int r;
@@ -2803,7 +2763,7 @@ __global__ void __launch_bounds__(TP_THREADS, 2) k_trsm_tcp(DevStruct s, const U
 // ---------------------------------------------------------------------------
 // Host launch wrappers (called from the driver with level lists in device memory)
 // ---------------------------------------------------------------------------
-static int sm_count() {
+int sm_count() {
     static int n = 0;
     if (n == 0) {
         int dev = 0;

@@ -1,0 +1,485 @@
+// FP64 updates on the 5th-generation tensor cores through exact integer slices
+// (tcgen05.mma kind::i8, 32-bit integer accumulators in tensor memory).
+//
+// The product C -= A B^T of an update task is formed from fixed-point operands
+// (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms
+// 59, 2012, with a common exponent per row): k_split_i8 scales every panel row
+// by a power of two, rounds it to 55 fractional bits below the row's largest
+// entry and cuts the integer into seven signed 8-bit digits (balanced base
+// 256).  Products of digits and their sums over up to I8_MAX_K columns are
+// exact in 32 bits; the digit products i, j with i + j <= 7 are kept (34 of
+// 49).  What is dropped -- 2^-64 of the largest products of a row pair, and the
+// rounding of entries smaller than 1/4 of their row's largest -- lies below the
+// rounding of the K additions that an FP64 accumulation of the same product
+// makes; the sums of the kept products are exact and are rounded once.  Rows
+// with a non-finite entry carry a NaN scale, so that it reaches the target.
+// Rounding relative to the row's largest entry asks for columns of like size:
+// the rows of a Cholesky factor are bounded by the diagonal of A, those of L in
+// LDL^T and LU are not (a small pivot makes a large column).  There column c is
+// scaled by h_c = 2^(half the exponent of the pivot), exactly: (L h)(L D / h)^T
+// and (L h)(U / h), the balance that Cholesky has.
+//
+// Why: the FP64 tensor cores (DMMA) multiply 64 x 2 flops per clock and SM, the
+// 8-bit ones 8192 x 2; 34 digit products per FP64 product are 3.8 times fewer
+// tensor-core cycles.  Rates measured are given at k_update_i8.
+//
+// Image of cblk k (bytes from i8_off[k]): digit p (0 the leading one), K block
+// kb of 32 columns, row group g of 8 panel rows at ((p * nkb + kb) * ng + g) *
+// I8_GROUP; inside a group the two 8 x 16-byte core matrices of the tensor
+// cores' K-major, no-swizzle layout.  ng = ceil(stride / 8) + 16, so that a
+// window of 16 row groups from any group of the panel stays inside the image.
+#include "device.cuh"
+#include "tcgen05.cuh"
+
+#include <algorithm>
+
+namespace pgpu {
+
+constexpr int I8_S = 7;                    // digits
+constexpr int I8_KB = 32;                  // columns per K block (one MMA step)
+constexpr int I8_GROUP = 256;              // bytes of 8 rows x 32 columns of one digit
+constexpr int I8_PIECE = 16 * I8_GROUP;    // one digit of a 128-row operand block
+constexpr int I8_STAGE = 2 * I8_S * I8_PIECE;
+constexpr int I8_STAGES = 3;
+constexpr size_t I8_SMEM = (size_t)I8_STAGES * I8_STAGE;
+constexpr int I8_THREADS = 320;            // 8 epilogue warps, producer, MMA issuer
+constexpr int I8_EPI = 256;
+constexpr int I8_BN = 128;
+constexpr int I8_TQ = 4;                   // tile-index ring
+constexpr int I8_MAX_K = 512;              // widest source: the low part of the sums stays within 2^50
+
+__host__ __device__ inline int i8_nkb(int nc) { return (nc + I8_KB - 1) / I8_KB; }
+__host__ __device__ inline int i8_ng(int st) { return (st + 7) / 8 + 16; }
+
+long long i8_image_bytes(int nc, int st) { return (long long)I8_S * i8_nkb(nc) * i8_ng(st) * I8_GROUP; }
+int i8_max_k() { return I8_MAX_K; }
+
+// ---------------------------------------------------------------------------
+// Digits of 32-row slabs (blockIdx.y) of 128-row panel slabs.  A lane holds a
+// row; the warps share its 16-column chunks.  The first pass finds the row's
+// largest magnitude, the second (the slab is in L1 / L2 by then) writes the
+// digits, 16 bytes per digit and chunk.  Column factors by `mode`: 0 none, 1 h_c,
+// 2 D_c / h_c, 3 1 / h_c, with D_c the pivot on the diagonal of panel Dp.  Bound
+// by HBM: 8 bytes read and 7 written per entry.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *__restrict__ slabs, const double *P,
+                                                  const double *Dp, const int64_t *__restrict__ i8_off,
+                                                  unsigned char *img, double *__restrict__ rscale, int mode) {
+    __shared__ double red[8][32];
+    __shared__ int badw[8][32];
+    __shared__ double colf[I8_MAX_K];
+    const SplitSlab sl = slabs[blockIdx.x];
+    const int k = sl.cblk;
+    const int nc = s.cb_lcol[k] - s.cb_fcol[k] + 1;
+    const int st = s.cb_stride[k];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pr = sl.r0 + 32 * blockIdx.y + lane;
+    if (sl.r0 + 32 * (int)blockIdx.y >= st) return;  // whole CTA
+    const int nkb = i8_nkb(nc), ng = i8_ng(st), nch = 2 * nkb;
+    const double *A = P + s.cb_coef[k] + pr;
+    const double *D = Dp + s.cb_coef[k];
+    auto load = [&](int ch, double (&v)[16]) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const int c = 16 * ch + j;
+            v[j] = (pr < st && c < nc) ? A[(size_t)c * st] : 0.0;
+        }
+        if (mode) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const int c = 16 * ch + j;
+                if (c < nc) v[j] *= colf[c];
+            }
+        }
+    };
+    auto pow2 = [](int e) { return __hiloint2double((e + 1023) << 20, 0); };
+    if (mode) {
+        for (int c = threadIdx.x; c < nc; c += 256) {
+            const double d = D[c + (size_t)c * st];
+            const int e = (__double2hiint(d) >> 20) & 0x7ff;
+            const int h = (e == 0 || e == 0x7ff) ? 0 : (e - 1023) / 2;  // zero and non-finite pivots: none
+            colf[c] = mode == 1 ? pow2(h) : (mode == 2 ? d * pow2(-h) : pow2(-h));
+        }
+        __syncthreads();
+    }
+    double m = 0.0;
+    int bad = 0;
+    for (int ch = warp; ch < nch; ch += 8) {
+        double v[16];
+        load(ch, v);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const double a = fabs(v[j]);
+            m = a > m ? a : m;
+            bad |= !(a <= 1.7976931348623157e308);
+        }
+    }
+    red[warp][lane] = m;
+    badw[warp][lane] = bad;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        m = red[w][lane] > m ? red[w][lane] : m;
+        bad |= badw[w][lane];
+    }
+    // row exponent: |a| < 127.375 / 128 * 2^ex, so that the leading digit fits 8
+    // bits after the carries of the balanced digits (at most 0.502 of it)
+    int ex = ((__double2hiint(m) >> 20) & 0x7ff) - 1022;
+    if (ex < -900) ex = -900;  // rows below 2^-900: absolute rounding
+    if (!bad && m >= 0.9951171875 * pow2(ex - 1) * 2.0) ex++;
+    const double mult = bad ? 0.0 : pow2(55 - ex);
+    if (warp == 0 && pr < st)
+        rscale[s.cb_rowidx[k] + pr] = bad ? __longlong_as_double(0x7ff8000000000000LL) : pow2(ex - 19);
+    if (pr >= 8 * ((st + 7) / 8)) return;
+    unsigned char *out = img + i8_off[k] + (size_t)(pr >> 3) * I8_GROUP + (pr & 7) * 16;
+    for (int ch = warp; ch < nch; ch += 8) {
+        double v[16];
+        load(ch, v);
+        uint32_t w[I8_S][4];
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            uint32_t lo[4], hi[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const long long q = bad ? 0 : __double2ll_rn(v[4 * g + j] * mult);
+                const unsigned long long t = (unsigned long long)(q + 0x808080808080LL);
+                lo[j] = (uint32_t)t;
+                hi[j] = (uint32_t)(t >> 32);
+            }
+            // byte b of the four values, by 4 x 4 byte transposes
+            const uint32_t l01a = __byte_perm(lo[0], lo[1], 0x5140), l23a = __byte_perm(lo[2], lo[3], 0x5140);
+            const uint32_t l01b = __byte_perm(lo[0], lo[1], 0x7362), l23b = __byte_perm(lo[2], lo[3], 0x7362);
+            const uint32_t h01a = __byte_perm(hi[0], hi[1], 0x5140), h23a = __byte_perm(hi[2], hi[3], 0x5140);
+            const uint32_t h01b = __byte_perm(hi[0], hi[1], 0x7362), h23b = __byte_perm(hi[2], hi[3], 0x7362);
+            w[6][g] = __byte_perm(l01a, l23a, 0x5410) ^ 0x80808080u;
+            w[5][g] = __byte_perm(l01a, l23a, 0x7632) ^ 0x80808080u;
+            w[4][g] = __byte_perm(l01b, l23b, 0x5410) ^ 0x80808080u;
+            w[3][g] = __byte_perm(l01b, l23b, 0x7632) ^ 0x80808080u;
+            w[2][g] = __byte_perm(h01a, h23a, 0x5410) ^ 0x80808080u;
+            w[1][g] = __byte_perm(h01a, h23a, 0x7632) ^ 0x80808080u;
+            w[0][g] = __byte_perm(h01b, h23b, 0x5410);
+        }
+        unsigned char *o = out + (size_t)(ch >> 1) * ng * I8_GROUP + (ch & 1) * 128;
+#pragma unroll
+        for (int p = 0; p < I8_S; p++)
+            *reinterpret_cast<uint4 *>(o + (size_t)p * nkb * ng * I8_GROUP) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The tile kernel: persistent, warp specialized, tiles from a device work queue
+// as in the FP32 engine.  128 x 128 tiles; the eight digit sums d = i + j do not
+// fit the 512 tensor-memory columns at once, so that a tile takes two passes
+// over K: first d = 4..7 (24 digit products, seven digits of each operand), kept
+// by the epilogue threads as 31-bit integers, then d = 0..3 (10 products, four
+// digits), added and scattered into the facing panel.  N = 128 rather than 64
+// with all sums resident: at N = 64 the tensor cores read shared memory faster
+// than it delivers (192 bytes a clock).
+// 100^3 Laplacian, B200, all updates of an FP64 factorization: 264 ms on DMMA
+// (k_update_dmma, 23 Tflop/s), 111 ms here (55 Tflop/s).  Bounds, 80^3: copies
+// alone 22.9 ms (L2 to shared memory, 35 bytes a clock and SM), products and
+// hand-offs alone 22.2 (tensor pipe 14.7), both without epilogue 24.0, with it
+// 31.8.  Slower: 16 or 8 epilogue warps that release the accumulators before
+// they scatter (33.1, 37.2: the registers spill), one polling lane per warp (34.7).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t i8_desc(uint32_t saddr) {
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(I8_GROUP >> 4) << 32) |
+           (1ull << 46);
+}
+// S8 x S8 -> S32, both operands K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t i8_idesc(int n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+__device__ __forceinline__ void i8_mma(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
+// The four digit sums of 8 columns, a[d] = accumulator d: sum of a[d] 2^(24 - 8 d)
+__device__ __forceinline__ void i8_load4(uint32_t taddr, long long (&z)[8]) {
+    int a[4][8];
+#pragma unroll
+    for (int d = 0; d < 4; d++) tmem_ld8(taddr + I8_BN * d, a[d]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        z[j] = (((long long)a[0][j] * 256 + a[1][j]) << 16) + ((long long)a[2][j] * 256 + a[3][j]);
+}
+__device__ __forceinline__ int i8_bar_or(int pred) {  // OR over the epilogue threads, which it also orders
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.red.or.pred q, 1, 256, p;\n\t"
+        "selp.b32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(pred)
+        : "memory");
+    return r;
+}
+
+template <int FACT>
+__global__ void __launch_bounds__(I8_THREADS, 1)
+    k_update_i8(DevStruct s, const UpdTile *__restrict__ tiles, int count, double *L, double *U,
+                const unsigned char *img0, const unsigned char *img1, const double *__restrict__ sc0,
+                const double *__restrict__ sc1, const int64_t *__restrict__ i8_off, int *queue, int *status) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t full[I8_STAGES], empty[I8_STAGES], tfull, tempty, tq_full[I8_TQ], tq_empty[I8_TQ];
+    __shared__ uint32_t tmem_sh;
+    __shared__ int ctab[2][I8_BN];
+    __shared__ double csc[2][I8_BN];
+    __shared__ int tq[I8_TQ];
+    if (*(volatile int *)status != 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
+                     "r"(4 * I8_BN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < I8_STAGES; i++) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        mbar_init(&tfull, 1);
+        mbar_init(&tempty, I8_EPI);
+        for (int i = 0; i < I8_TQ; i++) {
+            mbar_init(&tq_full[i], 1);
+            mbar_init(&tq_empty[i], 1 + I8_EPI);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_sh;
+    int late = 0;
+    if (warp == 8) {
+        if (lane == 0) {  // producer: claims tiles, loads their operands
+            uint32_t g = 0;
+            int next = atomicAdd(queue, 1);  // claimed one tile ahead
+            for (int j = 0; !late; j++) {
+                const int slot = j % I8_TQ;
+                if (j >= I8_TQ && !mbar_wait(&tq_empty[slot], ((j / I8_TQ) - 1) & 1)) {
+                    late = 1;
+                    break;
+                }
+                int t = next;
+                if (t >= count) t = -1;
+                else next = atomicAdd(queue, 1);
+                tq[slot] = t;
+                mbar_arrive(&tq_full[slot]);
+                if (t < 0) break;
+                const UpdTile tl = tiles[t];
+                const TaskDev tk = s.tasks[tl.task];
+                const int k = tk.src, K = s.cb_lcol[k] - s.cb_fcol[k] + 1, st = s.cb_stride[k];
+                const int nkb = i8_nkb(K), ng = i8_ng(st);
+                const int ga = ((tk.row0 + (tl.side ? tk.n : 0)) >> 3) + 16 * tl.mt, gb = (tk.row0 >> 3) + 16 * tl.nt;
+                const int nmma = (min(I8_BN, tk.row0 + tk.n - 8 * gb) + 15) & ~15;
+                const bool swap = (FACT == FACT_GETRF && tl.side == 1);
+                const unsigned char *iA = (swap ? img1 : img0) + i8_off[k];
+                const unsigned char *iB = ((FACT == FACT_POTRF) ? img0 : (swap ? img0 : img1)) + i8_off[k];
+                const size_t digit = (size_t)nkb * ng * I8_GROUP;
+                const uint32_t bbytes = (uint32_t)(nmma / 8) * I8_GROUP;
+                for (int pass = 0; pass < 2 && !late; pass++) {
+                    const int nd = pass ? 4 : I8_S;
+                    for (int kb = 0; kb < nkb; kb++, g++) {
+                        const int sidx = g % I8_STAGES;
+                        if (g >= I8_STAGES && !mbar_wait(&empty[sidx], ((g / I8_STAGES) - 1) & 1)) {
+                            late = 1;
+                            break;
+                        }
+                        unsigned char *sp = smem_raw + (size_t)sidx * I8_STAGE;
+                        mbar_expect_tx(&full[sidx], (uint32_t)nd * (I8_PIECE + bbytes));
+                        for (int p = 0; p < nd; p++) {
+                            bulk_g2s(sp + p * I8_PIECE, iA + p * digit + ((size_t)kb * ng + ga) * I8_GROUP, I8_PIECE,
+                                     &full[sidx]);
+                            bulk_g2s(sp + (I8_S + p) * I8_PIECE, iB + p * digit + ((size_t)kb * ng + gb) * I8_GROUP,
+                                     bbytes, &full[sidx]);
+                        }
+                    }
+                }
+            }
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {  // MMA issuer
+            const uint32_t sbase = smem_u32(smem_raw);
+            uint32_t g = 0, ph = 0;
+            for (int i = 0; !late; i++) {
+                const int slot = i % I8_TQ;
+                if (!mbar_wait(&tq_full[slot], (i / I8_TQ) & 1)) {
+                    late = 1;
+                    break;
+                }
+                const int t = tq[slot];
+                mbar_arrive(&tq_empty[slot]);
+                if (t < 0) break;
+                const UpdTile tl = tiles[t];
+                const TaskDev tk = s.tasks[tl.task];
+                const int nkb = i8_nkb(s.cb_lcol[tk.src] - s.cb_fcol[tk.src] + 1);
+                const int gb = (tk.row0 >> 3) + 16 * tl.nt;
+                const uint32_t idesc = i8_idesc((min(I8_BN, tk.row0 + tk.n - 8 * gb) + 15) & ~15);
+                for (int pass = 0; pass < 2 && !late; pass++, ph++) {
+                    if (ph > 0 && !mbar_wait(&tempty, (ph - 1) & 1)) {  // accumulators drained
+                        late = 1;
+                        break;
+                    }
+                    tc_fence_after();
+                    for (int kb = 0; kb < nkb; kb++, g++) {
+                        const int sidx = g % I8_STAGES;
+                        if (!mbar_wait(&full[sidx], (g / I8_STAGES) & 1)) {
+                            late = 1;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint64_t da = i8_desc(sbase + sidx * I8_STAGE);
+                        const uint64_t db = i8_desc(sbase + sidx * I8_STAGE + I8_S * I8_PIECE);
+                        if (pass == 0) {
+#pragma unroll
+                            for (int d = 4; d < 8; d++)
+#pragma unroll
+                                for (int p = d - 6 > 0 ? d - 6 : 0; p <= (d < 6 ? d : 6); p++)
+                                    i8_mma(tmem + I8_BN * (d - 4), da + p * (I8_PIECE >> 4), db + (d - p) * (I8_PIECE >> 4),
+                                           idesc, kb > 0 || p > (d - 6 > 0 ? d - 6 : 0));
+                        } else {
+#pragma unroll
+                            for (int d = 0; d < 4; d++)
+#pragma unroll
+                                for (int p = 0; p <= d; p++)
+                                    i8_mma(tmem + I8_BN * d, da + p * (I8_PIECE >> 4), db + (d - p) * (I8_PIECE >> 4), idesc,
+                                           kb > 0 || p > 0);
+                        }
+                        tc_commit(&empty[sidx]);
+                    }
+                    if (!late) tc_commit(&tfull);
+                }
+            }
+        }
+    } else {  // epilogue: warps w and w + 4 share 32 tile rows, 64 columns each
+        const int row = 32 * (warp & 3) + lane, cbase = 64 * (warp >> 2);
+        uint32_t ph = 0;
+        for (int i = 0;; i++) {
+            const int slot = i % I8_TQ;
+            if (i8_bar_or(!mbar_wait(&tq_full[slot], (i / I8_TQ) & 1))) {
+                late = 1;
+                break;
+            }
+            const int t = tq[slot];
+            mbar_arrive(&tq_empty[slot]);
+            if (t < 0) break;
+            const UpdTile tl = tiles[t];
+            const TaskDev tk = s.tasks[tl.task];
+            const int k = tk.src, f = tk.dst, b = i & 1;
+            const bool swap = (FACT == FACT_GETRF && tl.side == 1);
+            const double *scA = (swap ? sc1 : sc0) + s.cb_rowidx[k];
+            const double *scB = ((FACT == FACT_POTRF) ? sc0 : (swap ? sc0 : sc1)) + s.cb_rowidx[k];
+            const int *ridx = s.rowidx + s.cb_rowidx[k];
+            const int ra = tk.row0 + (tl.side ? tk.n : 0);
+            const int pr = 8 * ((ra >> 3) + 16 * tl.mt) + row, gb = (tk.row0 >> 3) + 16 * tl.nt;
+            const int nmma = (min(I8_BN, tk.row0 + tk.n - 8 * gb) + 15) & ~15;
+            if (tid < I8_BN) {  // target columns and their scales
+                const int pc = 8 * gb + tid;
+                const bool in = pc >= tk.row0 && pc < tk.row0 + tk.n;
+                ctab[b][tid] = in ? ridx[pc] - s.cb_fcol[f] : -1;
+                csc[b][tid] = in ? scB[pc] : 0.0;
+            }
+            int rr = -1;  // target row in the facing panel
+            double rs = 0.0;
+            if (pr >= ra && pr < tk.row0 + tk.m) {
+                const int g = ridx[pr];
+                int lo = s.cb_fblok[f], hi = s.cb_fblok[f + 1] - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (s.bk_frow[mid] <= g) lo = mid;
+                    else hi = mid - 1;
+                }
+                rr = s.bk_rowoff[lo] + (g - s.bk_frow[lo]);
+                rs = -scA[pr];
+            }
+            const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)cbase;
+            if (i8_bar_or(!mbar_wait(&tfull, ph & 1))) {
+                late = 1;
+                break;
+            }
+            tc_fence_after();
+            ph++;
+            int low[64];  // the sums d = 4..7 in units of 2^20 of the last digit's
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                if (cbase + 8 * q < nmma) {
+                    long long z[8];
+                    i8_load4(taddr + 8 * q, z);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) low[8 * q + j] = (int)((z[j] + (1 << 19)) >> 20);
+                }
+            }
+            tc_fence_before();
+            mbar_arrive(&tempty);
+            if (i8_bar_or(!mbar_wait(&tfull, ph & 1))) {
+                late = 1;
+                break;
+            }
+            tc_fence_after();
+            ph++;
+            double *Cp = (swap ? U : L) + s.cb_coef[f] + (rr >= 0 ? rr : 0);
+            const int stf = s.cb_stride[f];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                if (cbase + 8 * q < nmma) {
+                    long long z[8];
+                    i8_load4(taddr + 8 * q, z);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        // both integers to FP64 exactly (|z| < 2^51) by the offset of their magic exponents
+                        const double h = __longlong_as_double(z[j] + 0x4338000000000000LL) - 6755399441055744.0;
+                        const double l = __hiloint2double(0x43300000, low[8 * q + j] ^ 0x80000000) - 4503601774854144.0;
+                        const int cc = ctab[b][cbase + 8 * q + j];
+                        const double v = fma(l, 0x1p-12, h) * rs * csc[b][cbase + 8 * q + j];
+                        if (rr >= 0 && cc >= 0) atomicAdd(Cp + (size_t)cc * stf, v);
+                    }
+                }
+            }
+            tc_fence_before();
+            mbar_arrive(&tempty);
+        }
+    }
+    __syncwarp();
+    const int aborted = __syncthreads_or(late);
+    if (aborted && tid == 0) atomicExch(status, PGPU_STATUS_TIMEOUT);
+    tc_fence_after();
+    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(4 * I8_BN));
+}
+
+// ---------------------------------------------------------------------------
+void launch_split_i8(const DevStruct &s, const SplitSlab *slabs, int count, const double *P, const double *D,
+                     const int64_t *i8_off, unsigned char *img, double *rscale, int scale, cudaStream_t st) {
+    if (count <= 0) return;
+    k_split_i8<<<dim3(count, 4), 256, 0, st>>>(s, slabs, P, D, i8_off, img, rscale, scale);
+}
+template <int FACT>
+void launch_update_i8(const DevStruct &s, const UpdTile *tiles, int count, double *L, double *U,
+                      const unsigned char *img0, const unsigned char *img1, const double *sc0, const double *sc1,
+                      const int64_t *i8_off, int *queue, int *status, int sms, cudaStream_t st) {
+    if (count <= 0) return;
+    k_update_i8<FACT><<<std::min(count, sms), I8_THREADS, I8_SMEM, st>>>(s, tiles, count, L, U, img0, img1, sc0, sc1,
+                                                                         i8_off, queue, status);
+}
+cudaError_t set_i8_attrs() {
+    cudaError_t e = cudaSuccess;
+    for (auto k : {k_update_i8<FACT_POTRF>, k_update_i8<FACT_SYTRF>, k_update_i8<FACT_GETRF>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)I8_SMEM);
+    return e;
+}
+#define PGPU_INST_I8(F)                                                                                               \
+    template void launch_update_i8<F>(const DevStruct &, const UpdTile *, int, double *, double *,                    \
+                                      const unsigned char *, const unsigned char *, const double *, const double *,   \
+                                      const int64_t *, int *, int *, int, cudaStream_t);
+PGPU_INST_I8(FACT_POTRF)
+PGPU_INST_I8(FACT_SYTRF)
+PGPU_INST_I8(FACT_GETRF)
+
+}  // namespace pgpu
