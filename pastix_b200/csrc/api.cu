@@ -1179,6 +1179,14 @@ static int build_maps_and_lists(pastix_data_t *pd) {
     pd->trsm_tc_tiles.clear();
     pd->trsm_tiles32.clear();
     const int nsides = (fk == pgpu::FACT_GETRF) ? 2 : 1;
+    // TRSM row tiles of a cblk, an even number (the last one may be empty): a CTA may take two
+    auto row_tiles = [](std::vector<pgpu::RowTile> &list, idx_t k, idx_t nc, idx_t st) {
+        const idx_t bm = pgpu::trsm_tile_rows((int)nc);
+        for (idx_t r = nc; r < st; r += 2 * bm) {
+            list.push_back(pgpu::RowTile{(int)k, (int)r});
+            list.push_back(pgpu::RowTile{(int)k, (int)(r + bm)});
+        }
+    };
     for (idx_t k = 0; k < sv.cblknbr; k++) {
         const idx_t nc = sv.cb_lcol[k] - sv.cb_fcol[k] + 1, st = sv.cb_stride[k];
         if (pd->sp_off[k] < 0 || st <= nc || st * nc <= SMALL_PANEL_ELEMS || nc > 32 * pgpu::trinv_max_blocks())
@@ -1215,8 +1223,7 @@ static int build_maps_and_lists(pastix_data_t *pd) {
                 L.diag_maxnc = std::max<int>(L.diag_maxnc, (int)nc);
                 pd->dinv_total += pgpu::dinv_elems((int)nc, fk);
                 L.diag_smem_elems = std::max<size_t>(L.diag_smem_elems, (size_t)pgpu::diag_smem_elems((int)nc, fk));
-                int bm = pgpu::trsm_tile_rows((int)nc);
-                for (idx_t r = nc; r < st; r += bm) pd->trsm_tiles.push_back(pgpu::RowTile{(int)k, (int)r});
+                row_tiles(pd->trsm_tiles, k, nc, st);
                 if (st > nc) L.trsm_smem_elems = std::max<size_t>(L.trsm_smem_elems, (size_t)pgpu::trsm_smem_elems((int)nc));
                 if (st > nc) L.trsm_maxnc = std::max<int>(L.trsm_maxnc, (int)nc);
             }
@@ -1238,8 +1245,7 @@ static int build_maps_and_lists(pastix_data_t *pd) {
             const idx_t nc = sv.cb_lcol[k] - sv.cb_fcol[k] + 1, st = sv.cb_stride[k];
             if (st * nc <= SMALL_PANEL_ELEMS || st <= nc) continue;
             if (pd->ti_off[k] < 0) {
-                for (idx_t r = nc; r < st; r += pgpu::trsm_tile_rows((int)nc))
-                    pd->trsm_tiles32.push_back(pgpu::RowTile{(int)k, (int)r});
+                row_tiles(pd->trsm_tiles32, k, nc, st);
                 continue;
             }
             L.ti_maxnzb = std::max<int>(L.ti_maxnzb, (int)((nc + 31) / 32));

@@ -485,6 +485,7 @@ __global__ void __launch_bounds__(256) k_trsm(DevStruct s, const RowTile *__rest
     const int k = tl.cblk;
     const int nc = s.cb_lcol[k] - s.cb_fcol[k] + 1;
     const int st = s.cb_stride[k];
+    if (tl.r0 >= st) return;  // the tile that pads a cblk's pairs
     const int rows = min(TRSM_ROWS, st - tl.r0);
     const int ld = nc + 1;
     T *X = reinterpret_cast<T *>(smem_raw);  // TRSM_ROWS x nc, row major, ld
@@ -882,66 +883,113 @@ __global__ void __launch_bounds__(256) k_update_dmma(DevStruct s, const UpdTile 
 
 // ---------------------------------------------------------------------------
 // Off-diagonal TRSM on FP64 tensor cores (DMMA m8n8k4), X T = A for a tile of
-// 32 panel rows of a wide cblk, T the upper triangular factor of the diagonal
+// 8 RF panel rows of a wide cblk, T the upper triangular factor of the diagonal
 // block (L^T for POTRF, D L^T for SYTRF, U and L^T for the two GETRF sides),
-// as cpucblk_ztrsmsp (kernels/core_ztrsmsp.c:356).  The whole 32 x nc tile
-// stays in registers as 8 x 8 accumulator fragments: warp w owns the column
-// fragments w, w + 8, w + 16, ... (nc <= TD_MAXNC).  Column block j (32
-// columns) is solved with the inverted diagonal sub-block Z = T_jj^{-1} from
-// k_diag_large plus one residual correction, X_j = X0 + (A_j - X0 T_jj) Z
-// with X0 = A_j Z, then subtracted from the fragments to its right with T's
-// rows of block j read straight from the (L2-resident) diagonal block.
-// Storage may be FP32 (mixed precision); the arithmetic is FP64 throughout.
+// as cpucblk_ztrsmsp (kernels/core_ztrsmsp.c:356).  The whole tile stays in
+// registers as 8 x 8 accumulator fragments: warp w owns the column fragments w,
+// w + 8, w + 16, ... (nc <= TD_MAXNC).  Column block j (32 columns) is solved
+// with the inverted diagonal sub-block Z = T_jj^{-1} of the diagonal
+// factorization plus one residual correction, X_j = X0 + (A_j - X0 T_jj) Z with
+// X0 = A_j Z, then subtracted from the fragments to its right.
+// Z, T_jj and T's rows of block j + 1 are copied by cp.async into the second of
+// two shared-memory buffers while block j is worked on: read from L2 inside the
+// product loops they set its pace (54 us for a tile of 288 columns, four times
+// its DMMA time).  All levels of a factorization, FP64, B200: 32^3 elastic LDL^T
+// 7.0 -> 3.5 ms, 45x38x41 convection-diffusion LU 3.1 -> 1.9 ms, 100^3 Laplacian
+// 40.3 -> 33.5 ms (36.2 with single tiles; its DMMA work, the three products
+// with Z and T_jj included, takes 15 ms at the DGEMM rate), 20^3 Laplacian
+// 0.20 -> 0.10 ms.  RF = 4 where the tiles fill the SMs, RF = 2 (half the
+// products per step, twice the CTAs) where they do not.  G row tiles share a CTA
+// and its buffers, eight warps each with barriers of their own, so that with
+// G = 2 the products of one overlap the dependent steps of the other.  LDL^T
+// applies D to the rows of X.  Storage may be FP32 (mixed precision); the
+// arithmetic is FP64.
 // ---------------------------------------------------------------------------
 constexpr int TD_Q = 6;                 // column fragments per warp
 constexpr int TD_MAXNC = 8 * TD_Q * 8;  // 384 columns
 constexpr int TD_LDS = 36;              // shared row stride (doubles): 2 wavefronts per fragment load
-
-// T(a, b) of the upper triangular factor, a <= b < nc (callers guarantee it).
-template <typename T, int FACT>
-__device__ __forceinline__ double trsm_tval(const T *D, int st, int a, int b, int side) {
-    if (FACT == FACT_POTRF) return (double)D[b + (size_t)a * st];
-    if (FACT == FACT_SYTRF) {
-        const double da = (double)D[a + (size_t)a * st];
-        return (a == b) ? da : da * (double)D[b + (size_t)a * st];
-    }
-    if (side == 0) return (double)D[a + (size_t)b * st];
-    return (a == b) ? 1.0 : (double)D[b + (size_t)a * st];
+constexpr int TD_LDZ = 36;
+// One buffer: Z, T_jj (32 x 32) and the first `cap` columns of the strip of T right of block j, element (a, b) at
+// a * (cap + 4) + b (a row stride of 4 mod 16 doubles: fragment loads without bank conflicts).  The cap holds the
+// strips of FP64 blocks up to 320 columns; wider ones read the rest from global memory.
+__host__ __device__ inline int td_buf(int cap) { return 2 * 32 * TD_LDZ + 32 * (cap + 4); }
+inline int td_cap(int maxnc, int tsize) {
+    const int w = ((maxnc > 32 ? maxnc - 32 : 0) + 15) / 16 * 16;
+    return std::min(w, tsize == 8 ? 288 : 352);
 }
+inline size_t trsm_dmma_smem(int cap, int tsize) { return 2 * (size_t)td_buf(cap) * tsize; }
 
-template <typename T, int FACT>
-__global__ void __launch_bounds__(256, 2) k_trsm_dmma(DevStruct s, const RowTile *__restrict__ tiles, T *L, T *U,
-                                                       const T *__restrict__ dinv) {
-    __shared__ double As[32 * TD_LDS], Xs[32 * TD_LDS], Rs[32 * TD_LDS];
-    const RowTile tl = tiles[blockIdx.x];
+template <typename T, int FACT, int RF, int G>
+__global__ void __launch_bounds__(256 * G, RF == 4 ? 1 : 2) k_trsm_dmma(DevStruct s, const RowTile *__restrict__ tiles,
+                                                                    T *L, T *U, const T *__restrict__ dinv, int cap) {
+    constexpr int ROWS = 8 * RF, SPLIT = 4 / RF, NF = RF / 2;  // NF: 8 x 8 fragments of the 32-column block per warp
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double Ash[G][ROWS * TD_LDS], Xsh[G][ROWS * TD_LDS];
+    __shared__ double ds[TD_MAXNC];
+    pdl_wait();
+    const int tid = threadIdx.x, lane = tid & 31, grp = tid >> 8, warp = (tid >> 5) & 7;
+    RowTile tl = tiles[G * (blockIdx.x / SPLIT) + grp];  // the G tiles of a CTA belong to one cblk
+    tl.r0 += ROWS * (blockIdx.x % SPLIT);
+    double *As = Ash[grp], *Xs = Xsh[grp];
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + grp) : "memory"); };
     const int side = blockIdx.y;
     const int k = tl.cblk;
     const int nc = s.cb_lcol[k] - s.cb_fcol[k] + 1;
     const int st = s.cb_stride[k];
-    const int rows = min(32, st - tl.r0);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (G == 1 && tl.r0 >= st) return;  // whole CTA
+    const int rows = min(ROWS, st - tl.r0);  // none for the tile that pads a pair
     const int g = lane >> 2, t4 = lane & 3;
     const T *D = L + s.cb_coef[k];
     T *A = ((FACT == FACT_GETRF && side == 1) ? U : L) + s.cb_coef[k] + tl.r0;
     const int nzb = (nc + 31) / 32;
     const int ncf = (nc + 7) / 8;
     const T *gZ = dinv + s.cb_dinv[k] + (size_t)(side ? nzb : 0) * 1024;
+    const int ldt = cap + 4;
+    T *buf = reinterpret_cast<T *>(smem_raw);
+    const bool trans = (FACT == FACT_GETRF && side == 0);  // T = U, stored by columns; else T = L^T
+    auto cp = [](T *d, const T *p) {
+        if (sizeof(T) == 8) cp_async8(d, p, true);
+        else cp_async4(d, p, true);
+    };
+    auto prefetch = [&](int j) {
+        if (j < nzb) {
+            const int jb = 32 * j, w = min(nc - jb, 32 + cap);  // columns of T from block j on
+            T *Zs = buf + (j & 1) * td_buf(cap), *Tj = Zs + 32 * TD_LDZ, *Ts = Tj + 32 * TD_LDZ;
+            for (int e = tid; e < 1024; e += 256 * G) cp(Zs + (e >> 5) * TD_LDZ + (e & 31), gZ + (size_t)j * 1024 + e);
+            const int nb = min(32, w);
+            if (trans) {  // element (a, b) at D[a + b st]: lanes over a
+                for (int b = tid >> 5; b < w; b += 8 * G)
+                    if (lane < nb) cp(b < 32 ? Tj + lane * TD_LDZ + b : Ts + lane * ldt + b - 32, D + jb + lane + (size_t)(jb + b) * st);
+            } else {  // element (a, b) at D[b + a st]: lanes over b
+                for (int a = tid >> 5; a < nb; a += 8 * G)
+                    for (int b = lane; b < w; b += 32)
+                        cp(b < 32 ? Tj + a * TD_LDZ + b : Ts + a * ldt + b - 32, D + jb + b + (size_t)(jb + a) * st);
+            }
+        }
+        cp_async_commit();
+    };
+    prefetch(0);
+    prefetch(1);
+    if (FACT == FACT_SYTRF)
+        for (int i = tid; i < 32 * nzb; i += 256 * G) ds[i] = i < nc ? (double)D[i + (size_t)i * st] : 0.0;
 
-    double acc[4][TD_Q][2];
+    double acc[RF][TD_Q][2];
 #pragma unroll
     for (int q = 0; q < TD_Q; q++) {
         const int c0 = 8 * (warp + 8 * q) + 2 * t4;
 #pragma unroll
-        for (int rf = 0; rf < 4; rf++) {
+        for (int rf = 0; rf < RF; rf++) {
             const int r = 8 * rf + g;
 #pragma unroll
             for (int e = 0; e < 2; e++)
                 acc[rf][q][e] = (r < rows && c0 + e < nc) ? (double)A[r + (size_t)(c0 + e) * st] : 0.0;
         }
     }
-    const int orf = warp >> 1, ocf = 2 * (warp & 1);  // this warp's fragments of the 32 x 32 block solve
+    // this warp's fragments of the block solve: row fragment orf, column fragments ocf .. ocf + NF - 1
+    const int orf = warp / (4 / NF), ocf = NF * (warp % (4 / NF));
     for (int j = 0; j < nzb; j++) {
-        const int jb = 32 * j;
+        const int jb = 32 * j, nb = min(32, nc - jb);
+        const T *Zs = buf + (j & 1) * td_buf(cap), *Tj = Zs + 32 * TD_LDZ, *Ts = Tj + 32 * TD_LDZ;
         // i. the owners of block j hand their fragments over to shared memory
 #pragma unroll
         for (int q = 0; q < TD_Q; q++) {
@@ -949,99 +997,116 @@ __global__ void __launch_bounds__(256, 2) k_trsm_dmma(DevStruct s, const RowTile
             if ((cf >> 2) == j) {
                 const int cc = 8 * (cf & 3) + 2 * t4;
 #pragma unroll
-                for (int rf = 0; rf < 4; rf++) {
+                for (int rf = 0; rf < RF; rf++) {
                     As[(8 * rf + g) * TD_LDS + cc] = acc[rf][q][0];
                     As[(8 * rf + g) * TD_LDS + cc + 1] = acc[rf][q][1];
                 }
             }
         }
+        cp_async_wait<1>();
         __syncthreads();
-        const T *Zj = gZ + (size_t)j * 1024;
-        double x0[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        // P (this warp's fragments) += src Z, two chains
+        auto times_z = [&](const double *src, double (&x)[NF][2]) {
+            double y[NF][2];
+#pragma unroll
+            for (int c = 0; c < NF; c++) y[c][0] = y[c][1] = 0.0;
+#pragma unroll
+            for (int ks = 0; ks < 8; ks += 2) {
+                const double a0 = src[(8 * orf + g) * TD_LDS + 4 * ks + t4], a1 = src[(8 * orf + g) * TD_LDS + 4 * ks + 4 + t4];
+#pragma unroll
+                for (int c = 0; c < NF; c++) {
+                    dmma884(x[c][0], x[c][1], a0, (double)Zs[(4 * ks + t4) * TD_LDZ + 8 * (ocf + c) + g]);
+                    dmma884(y[c][0], y[c][1], a1, (double)Zs[(4 * ks + 4 + t4) * TD_LDZ + 8 * (ocf + c) + g]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < NF; c++) {
+                x[c][0] += y[c][0];
+                x[c][1] += y[c][1];
+            }
+        };
         // ii-a. X0 = A_j Z
+        double x0[NF][2];
 #pragma unroll
-        for (int ks = 0; ks < 8; ks++) {
-            const double a = As[(8 * orf + g) * TD_LDS + 4 * ks + t4];
+        for (int c = 0; c < NF; c++) x0[c][0] = x0[c][1] = 0.0;
+        times_z(As, x0);
 #pragma unroll
-            for (int c = 0; c < 2; c++)
-                dmma884(x0[c][0], x0[c][1], a, (double)Zj[(4 * ks + t4) * 32 + 8 * (ocf + c) + g]);
-        }
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
+        for (int c = 0; c < NF; c++) {
             Xs[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4] = x0[c][0];
             Xs[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4 + 1] = x0[c][1];
         }
-        __syncthreads();
-        // ii-b. R = A_j - X0 T_jj
-        double rr[2][2];
+        group_sync();
+        // ii-b. R = A_j - X0 T_jj, in place of A_j (a thread reads and writes the same entries)
+        double rr[NF][2], r1[NF][2];
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
+        for (int c = 0; c < NF; c++) {
             rr[c][0] = As[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4];
             rr[c][1] = As[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4 + 1];
+            r1[c][0] = r1[c][1] = 0.0;
         }
 #pragma unroll
         for (int ks = 0; ks < 8; ks++) {
-            const double a = -Xs[(8 * orf + g) * TD_LDS + 4 * ks + t4];
-            const int ta = jb + 4 * ks + t4;
+            const int ta = 4 * ks + t4;
+            double a = -Xs[(8 * orf + g) * TD_LDS + ta];
+            if (FACT == FACT_SYTRF) a *= ds[jb + ta];
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const int tb = jb + 8 * (ocf + c) + g;
-                const double b = (ta <= tb && tb < nc) ? trsm_tval<T, FACT>(D, st, ta, tb, side) : 0.0;
-                dmma884(rr[c][0], rr[c][1], a, b);
+            for (int c = 0; c < NF; c++) {
+                const int tb = 8 * (ocf + c) + g;
+                double b = (ta <= tb && tb < nb) ? (double)Tj[ta * TD_LDZ + tb] : 0.0;
+                // unit triangles: LDL^T's L, and the L^T of the LU's U side
+                if ((FACT == FACT_SYTRF || (FACT == FACT_GETRF && side == 1)) && ta == tb && tb < nb) b = 1.0;
+                if (ks & 1) dmma884(r1[c][0], r1[c][1], a, b);
+                else dmma884(rr[c][0], rr[c][1], a, b);
             }
         }
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-            Rs[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4] = rr[c][0];
-            Rs[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4 + 1] = rr[c][1];
+        for (int c = 0; c < NF; c++) {
+            As[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4] = rr[c][0] + r1[c][0];
+            As[(8 * orf + g) * TD_LDS + 8 * (ocf + c) + 2 * t4 + 1] = rr[c][1] + r1[c][1];
         }
-        __syncthreads();
-        // ii-c. X_j = X0 + R Z, to shared memory and to the panel
-#pragma unroll
-        for (int ks = 0; ks < 8; ks++) {
-            const double a = Rs[(8 * orf + g) * TD_LDS + 4 * ks + t4];
-#pragma unroll
-            for (int c = 0; c < 2; c++)
-                dmma884(x0[c][0], x0[c][1], a, (double)Zj[(4 * ks + t4) * 32 + 8 * (ocf + c) + g]);
-        }
+        group_sync();
+        // ii-c. X_j = X0 + R Z, to the panel and (times D for LDL^T) to shared memory
+        times_z(As, x0);
         {
             const int r = 8 * orf + g;
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
+            for (int c = 0; c < NF; c++) {
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const int cc = 8 * (ocf + c) + 2 * t4 + e;
-                    Xs[r * TD_LDS + cc] = x0[c][e];
+                    Xs[r * TD_LDS + cc] = FACT == FACT_SYTRF ? x0[c][e] * ds[jb + cc] : x0[c][e];
                     if (r < rows && jb + cc < nc) A[r + (size_t)(jb + cc) * st] = (T)x0[c][e];
                 }
             }
         }
-        __syncthreads();
+        group_sync();
         // iii. fragments right of block j: acc -= X_j T(block j rows, their columns)
         if (4 * j + 4 < ncf) {
-#pragma unroll 2
+#pragma unroll
             for (int ks = 0; ks < 8; ks++) {
-                const int ta = jb + 4 * ks + t4;
-                double a[4];
+                double a[RF];
 #pragma unroll
-                for (int rf = 0; rf < 4; rf++) a[rf] = -Xs[(8 * rf + g) * TD_LDS + 4 * ks + t4];
-                double b[TD_Q];
-#pragma unroll
-                for (int q = 0; q < TD_Q; q++) {
-                    const int cf = warp + 8 * q;
-                    const int tb = 8 * cf + g;
-                    b[q] = (cf >= 4 * j + 4 && ta < nc && tb < nc) ? trsm_tval<T, FACT>(D, st, ta, tb, side) : 0.0;
-                }
+                for (int rf = 0; rf < RF; rf++) a[rf] = -Xs[(8 * rf + g) * TD_LDS + 4 * ks + t4];
 #pragma unroll
                 for (int q = 0; q < TD_Q; q++) {
                     const int cf = warp + 8 * q;
                     if (cf >= 4 * j + 4 && cf < ncf) {
+                        const int tb = 8 * cf + g;
+                        double b = 0.0;
+                        if (8 * cf + 8 - jb - 32 <= cap) {
+                            if (tb < nc) b = (double)Ts[(4 * ks + t4) * ldt + tb - jb - 32];
+                        } else if (tb < nc) {
+                            const int ta = jb + 4 * ks + t4;
+                            b = (double)(trans ? D[ta + (size_t)tb * st] : D[tb + (size_t)ta * st]);
+                        }
 #pragma unroll
-                        for (int rf = 0; rf < 4; rf++) dmma884(acc[rf][q][0], acc[rf][q][1], a[rf], b[q]);
+                        for (int rf = 0; rf < RF; rf++) dmma884(acc[rf][q][0], acc[rf][q][1], a[rf], b);
                     }
                 }
             }
         }
+        __syncthreads();  // the buffer may be refilled
+        prefetch(j + 2);
     }
 }
 
@@ -2816,11 +2881,19 @@ template <typename T, int FACT>
 void launch_trsm(const DevStruct &s, const RowTile *tiles, int count, int maxnc, size_t smem, T *L, T *U,
                  const T *dinv, cudaStream_t st) {
     if (count <= 0) return;
-    dim3 grid(count, FACT == FACT_GETRF ? 2 : 1);
-    if (maxnc <= TD_MAXNC)
-        k_trsm_dmma<T, FACT><<<grid, 256, 0, st>>>(s, tiles, L, U, dinv);
+    const int sides = FACT == FACT_GETRF ? 2 : 1, nsm = sm_count();
+    const int cap = td_cap(maxnc, (int)sizeof(T));
+    const size_t sm = trsm_dmma_smem(cap, (int)sizeof(T));
+    // pairs of 32-row tiles where they fill the SMs, 16-row tiles while these fit one
+    // wave, single 32-row tiles between
+    if (maxnc > TD_MAXNC)
+        launch_k(k_trsm<T, FACT>, dim3(count, sides), 256, smem, st, s, tiles, L, U, dinv);
+    else if (count / 2 * sides >= nsm)
+        launch_k(k_trsm_dmma<T, FACT, 4, 2>, dim3(count / 2, sides), dim3(512), sm, st, s, tiles, L, U, dinv, cap);
+    else if (2 * count * sides <= nsm)
+        launch_k(k_trsm_dmma<T, FACT, 2, 1>, dim3(2 * count, sides), dim3(256), sm, st, s, tiles, L, U, dinv, cap);
     else
-        launch_k(k_trsm<T, FACT>, grid, 256, smem, st, s, tiles, L, U, dinv);
+        launch_k(k_trsm_dmma<T, FACT, 4, 1>, dim3(count, sides), dim3(256), sm, st, s, tiles, L, U, dinv, cap);
 }
 
 template <typename T, int FACT>
@@ -2943,6 +3016,9 @@ cudaError_t set_smem_attrs(size_t, size_t, size_t) {
     if ((e = opt_in_smem(k_panel_small<T, FACT>)) != cudaSuccess) return e;
     if ((e = opt_in_smem(k_diag_large<T, FACT>)) != cudaSuccess) return e;
     if ((e = opt_in_smem(k_trsm<T, FACT>)) != cudaSuccess) return e;
+    if ((e = opt_in_smem(k_trsm_dmma<T, FACT, 2, 1>)) != cudaSuccess) return e;
+    if ((e = opt_in_smem(k_trsm_dmma<T, FACT, 4, 1>)) != cudaSuccess) return e;
+    if ((e = opt_in_smem(k_trsm_dmma<T, FACT, 4, 2>)) != cudaSuccess) return e;
     if ((e = opt_in_smem(k_diag_dmma<T, FACT>)) != cudaSuccess) return e;
     if ((e = opt_in_smem(k_diag_cluster<T, FACT>)) != cudaSuccess) return e;
     if constexpr (sizeof(T) == 8) {
