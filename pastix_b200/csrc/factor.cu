@@ -1763,34 +1763,39 @@ __global__ void __launch_bounds__(256, 1) k_diag_dmma(DevStruct s, const int *__
 // memory, so the step is bound by the owner's factorization and the cluster
 // barrier rather than by L2 round trips.
 // ---------------------------------------------------------------------------
-constexpr int DC = 8;                      // CTAs per cluster
+// CTAs per cluster: 8, or 16 (above the portable size) for LU blocks wider than
+// 288 columns: LU keeps whole columns, and two panels of such a block do not fit
+// one CTA next to the static buffers.  64^3 convection-diffusion, levels of one or
+// two such blocks: 680..990 us on one CTA each (k_diag_dmma), ~420 us on 16;
+// the diagonal blocks of the factorization 20.2 -> 15.8 ms.
+constexpr int DC_MAX = 16;
 constexpr int DC_MIN_NC = 96;              // narrower blocks stay on one CTA
 // dynamic shared memory next to the static ~37 KB
 __host__ __device__ constexpr long long dc_max_smem(int) { return 180 * 1024LL; }
-constexpr int DC_SLOTS = (DG_MAXNC / 32 + DC - 1) / DC;  // panels one CTA can own (nc <= DG_MAXNC)
+constexpr int dc_slots(int dc) { return (DG_MAXNC / 32 + dc - 1) / dc; }  // panels one CTA can own (nc <= DG_MAXNC)
 // POTRF / SYTRF: every finished panel is also written (FP64, column-major nc x nc,
 // from its top row down) to a per-cblk area of global memory, from which the
 // other CTAs read it for their updates: eight CTAs reading one CTA's shared
 // memory at once through the cluster are bound by that one SM, while L2 serves
 // them in parallel.
 constexpr size_t DC_SCR_DOUBLES = (size_t)DG_MAXNC * DG_MAXNC;
-constexpr int DC_MAX_CLUSTERS = 160 / DC;  // cblks of one launch: count * DC <= SM count
+constexpr int DC_MAX_CLUSTERS = 160 / 8;  // cblks of one launch: count * 8 <= SM count
 
 __host__ __device__ inline int dc_lo(int p, int fact) { return fact == FACT_GETRF ? 0 : 32 * p; }
-// Shared memory (doubles) of the panels CTA `rank` owns for a block of width nc.
-__host__ __device__ inline long long dc_panel_doubles(int nc, int fact, int rank) {
+// Shared memory (doubles) of the panels CTA 0, which holds the most, owns for a block of width nc.
+__host__ __device__ inline long long dc_panel_doubles(int nc, int fact, int dc) {
     const int np = (nc + 31) / 32;
     long long n = 0;
-    for (int p = rank; p < np; p += DC) n += (long long)(nc - dc_lo(p, fact)) * DG_LD;
+    for (int p = 0; p < np; p += dc) n += (long long)(nc - dc_lo(p, fact)) * DG_LD;
     return n;
 }
 // GETRF: the inverted (L_pp)^T of each panel a CTA factors, read by the other
 // CTAs, one slot per panel it owns, ahead of the panels
-__host__ __device__ inline long long dc_zs1_doubles(int fact) {
-    return fact == FACT_GETRF ? (long long)DC_SLOTS * 32 * DG_LD : 0;
+__host__ __device__ inline long long dc_zs1_doubles(int fact, int dc) {
+    return fact == FACT_GETRF ? (long long)dc_slots(dc) * 32 * DG_LD : 0;
 }
-__host__ __device__ inline long long diag_cluster_smem_bytes(int nc, int fact) {
-    return 8 * (dc_zs1_doubles(fact) + dc_panel_doubles(nc, fact, 0));  // CTA 0 holds the most
+__host__ __device__ inline long long diag_cluster_smem_bytes(int nc, int fact, int dc) {
+    return 8 * (dc_zs1_doubles(fact, dc) + dc_panel_doubles(nc, fact, dc));
 }
 
 // Cluster-scope flag of one CTA, read from another CTA of the cluster.
@@ -1819,7 +1824,7 @@ __device__ __forceinline__ bool dc_wait(uint32_t addr, int target) {
     return true;
 }
 
-template <typename T, int FACT>
+template <typename T, int FACT, int DC>
 __global__ void __cluster_dims__(DC, 1, 1) __launch_bounds__(256, 1)
     k_diag_cluster(DevStruct s, const int *__restrict__ list, T *L, T *U, T *dinv, FactParams fp) {
     pdl_wait();  // the kernel ahead in the stream has ended (programmatic dependent launch)
@@ -1828,7 +1833,7 @@ __global__ void __cluster_dims__(DC, 1, 1) __launch_bounds__(256, 1)
     // GETRF: inverted (L_pp)^T of each panel factored here (read by the other CTAs
     // for U_pq), one slot per panel; then this CTA's panels, one after the other
     double *Zs1 = reinterpret_cast<double *>(smem_raw);
-    double *Wl = Zs1 + dc_zs1_doubles(FACT);
+    double *Wl = Zs1 + dc_zs1_doubles(FACT, DC);
     __shared__ double Zs0[32 * DG_LD];                   // inverted top block of the panel being factored here
     __shared__ __align__(16) double Sx[8][8 * DG_LD];  // also the published steps of the top block's factorization
     __shared__ double Tb[32 * DG_LD];                    // the top block being factored
@@ -2856,6 +2861,28 @@ void launch_panel_small(const DevStruct &s, const int *list, int count, size_t s
     launch_k(k_panel_small<T, FACT>, count, 128, smem, st, s, list, L, U, fp);
 }
 
+// 16-CTA clusters of the LU kernel that the current device runs at once (0: none), for a
+// launch with `smem` dynamic bytes per CTA.
+template <typename T>
+static int dc16_clusters(size_t smem) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(DC_MAX);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = DC_MAX;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_diag_cluster<T, FACT_GETRF, DC_MAX>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 template <typename T, int FACT>
 void launch_diag_large(const DevStruct &s, const int *list, int count, int maxnc, size_t smem, T *L, T *U, T *dinv,
                        const FactParams &fp, cudaStream_t st) {
@@ -2867,11 +2894,20 @@ void launch_diag_large(const DevStruct &s, const int *list, int count, int maxnc
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             nsm = 1;
     }
-    const long long csm = diag_cluster_smem_bytes(maxnc, FACT);
-    if (maxnc <= DG_MAXNC && maxnc >= DC_MIN_NC && (long long)count * DC <= nsm && count <= DC_MAX_CLUSTERS &&
-        csm <= dc_max_smem(FACT))
-        launch_k(k_diag_cluster<T, FACT>, count * DC, 256, (size_t)csm, st, s, list, L, U, dinv, fp);
-    else if (maxnc <= DG_MAXNC)
+    const bool fits = maxnc <= DG_MAXNC && maxnc >= DC_MIN_NC;
+    const long long csm = diag_cluster_smem_bytes(maxnc, FACT, 8);
+    if (fits && (long long)count * 8 <= nsm && count <= DC_MAX_CLUSTERS && csm <= dc_max_smem(FACT)) {
+        launch_k(k_diag_cluster<T, FACT, 8>, count * 8, 256, (size_t)csm, st, s, list, L, U, dinv, fp);
+        return;
+    }
+    if constexpr (FACT == FACT_GETRF) {
+        const long long csm16 = diag_cluster_smem_bytes(maxnc, FACT, DC_MAX);
+        if (fits && csm16 <= dc_max_smem(FACT) && count <= dc16_clusters<T>((size_t)csm16)) {
+            launch_k(k_diag_cluster<T, FACT, DC_MAX>, count * DC_MAX, 256, (size_t)csm16, st, s, list, L, U, dinv, fp);
+            return;
+        }
+    }
+    if (maxnc <= DG_MAXNC)
         launch_k(k_diag_dmma<T, FACT>, count, 256, (size_t)diag_dmma_smem_bytes(maxnc), st, s, list, L, U, dinv, fp);
     else
         launch_k(k_diag_large<T, FACT>, count, 256, smem, st, s, list, L, U, dinv, fp);
@@ -3020,7 +3056,12 @@ cudaError_t set_smem_attrs(size_t, size_t, size_t) {
     if ((e = opt_in_smem(k_trsm_dmma<T, FACT, 4, 1>)) != cudaSuccess) return e;
     if ((e = opt_in_smem(k_trsm_dmma<T, FACT, 4, 2>)) != cudaSuccess) return e;
     if ((e = opt_in_smem(k_diag_dmma<T, FACT>)) != cudaSuccess) return e;
-    if ((e = opt_in_smem(k_diag_cluster<T, FACT>)) != cudaSuccess) return e;
+    if ((e = opt_in_smem(k_diag_cluster<T, FACT, 8>)) != cudaSuccess) return e;
+    if constexpr (FACT == FACT_GETRF) {
+        if ((e = opt_in_smem(k_diag_cluster<T, FACT, DC_MAX>)) != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(k_diag_cluster<T, FACT, DC_MAX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+    }
     if constexpr (sizeof(T) == 8) {
         if ((e = opt_in_smem(k_update_dmma<FACT>)) != cudaSuccess) return e;
     } else {

@@ -1,6 +1,7 @@
 """Off-diagonal triangular solves of the FP64 factorization at the edges of their
 tiles: blocks of 33 to 484 columns, and panels whose numbers of rows leave
-partial tiles and unpaired ones, in levels with few and with many tiles.
+partial tiles and unpaired ones, in levels with few and with many tiles.  The
+LU case of 306 columns takes the 16-CTA clusters of the diagonal blocks.
 
 Factors against the oracle's, entry sums of at most n products: n u = 6e-13.
 """
@@ -17,13 +18,14 @@ from test_gpu_parity import _mask_compare
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("fact", ["POTRF", "SYTRF", "GETRF"])
-@pytest.mark.parametrize("grid,bs", [((13, 13, 29), (33, 34)), ((9, 10, 60), (80, 90)), ((22, 21, 14), (300, 330)),
-                                     ((21, 22, 23), (300, 384)), ((40, 41, 3), (40, 64))])
+SMALL = [((13, 13, 20), (33, 34)), ((9, 10, 40), (80, 90)), ((40, 31, 3), (40, 64))]
+CASES = [(f, g, b) for f in ("POTRF", "SYTRF", "GETRF") for g, b in SMALL]
+CASES += [("POTRF", (21, 22, 23), (300, 384)), ("GETRF", (18, 17, 19), (300, 330)), ("SYTRF", (18, 18, 18), (320, 330))]
+
+
+@pytest.mark.parametrize("fact,grid,bs", CASES)
 def test_factor_edges(lib, oracle_mod, fact, grid, bs):
-    A = gen.laplacian7(*grid) if fact != "GETRF" else gen.convdiff27(*[max(3, g * 3 // 4) for g in grid])
-    if fact == "GETRF":
-        grid = tuple(max(3, g * 3 // 4) for g in grid)
+    A = gen.convdiff27(*grid) if fact == "GETRF" else gen.laplacian7(*grid)
     pd, S, info = analyse(A, grid, fact, min_bs=bs[0], max_bs=bs[1])
     px.task_numfact(pd, S)
     Lg, Ug = px.get_coeftab(pd, with_u=(fact == "GETRF"))
