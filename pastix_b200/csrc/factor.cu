@@ -66,147 +66,236 @@ __global__ void k_fill_coef(int64_t nnz, const double *__restrict__ vals, const 
 }
 
 // ---------------------------------------------------------------------------
-// Narrow cblks: whole panel (and U^T panel for LU) in shared memory,
-// right-looking column sweep over the width.  Column c: pivot, scale the
-// column below the diagonal, rank-1 update of the remaining columns on all
-// panel rows.  This is potf2/getf2/sytf2 on the diagonal block fused with the
-// off-diagonal TRSM.
+// Narrow cblks (at most 64 columns): whole panel (and U^T panel for LU) in
+// shared memory, factored, solved and sent on by one CTA of 128 threads.
+//   1. warp 0 factors the diagonal block, left looking, a row per lane (two
+//      above 32 columns): potf2 / getf2 / sytf2.  The other warps meanwhile find
+//      where the rows of each off-diagonal blok land in the cblks it updates.
+//   2. Every row below is solved by one thread, four columns at a time; no row
+//      waits for another.
+//   3. The updates of every task of the cblk (core_zgemmsp_2d2d) are formed from
+//      the panel in shared memory, one row and four columns per thread, and
+//      scattered into the facing panels with reductions.
+// Bound by latency: the leaves are thousands of such panels, the levels above
+// hold few.  Against a right-looking sweep with three barriers per column over
+// the whole panel and row tables built task by task, all levels of an FP64
+// factorization, B200: 20^3 Laplacian 0.25 -> 0.12 ms, 512^2 diffusion 0.75 ->
+// 0.42 ms, 32^3 elastic LDL^T 0.39 -> 0.17 ms, 100^3 Laplacian 1.40 -> 0.96 ms.
 // ---------------------------------------------------------------------------
-constexpr int PS_FB_CACHE = 512;  // facing bloks whose first rows k_panel_small keeps in shared memory
-// Shared memory of k_panel_small: the panel (twice for GETRF) and its int tables.
+constexpr int PS_THREADS = 128;
+constexpr int PS_BLOKS = 128;   // off-diagonal bloks whose targets are kept at a time
+constexpr int PS_PAIRS = 1024;  // (blok, later blok) pairs whose row shifts are kept at a time
+// Shared memory of k_panel_small: the panel (twice for GETRF), reciprocal pivots and the tables.
 __host__ __device__ inline long long panel_small_smem_bytes(long long panel_elems, int tsize, int maxst) {
-    return panel_elems * tsize + 4LL * (2 * maxst + 2 * PS_FB_CACHE);
+    return PS_BLOKS * 12LL + (panel_elems + 64) * tsize + 4LL * (maxst + PS_PAIRS);
 }
 
 template <typename T, int FACT>
-__global__ void __launch_bounds__(256) k_panel_small(DevStruct s, const int *__restrict__ list, T *L, T *U,
-                                                      FactParams fp) {
+__global__ void __launch_bounds__(PS_THREADS) k_panel_small(DevStruct s, const int *__restrict__ list, T *L, T *U,
+                                                             FactParams fp) {
     pdl_wait();  // the kernel ahead in the stream has ended (programmatic dependent launch)
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *P = reinterpret_cast<T *>(smem_raw);
     const int k = list[blockIdx.x];
     const int nc = s.cb_lcol[k] - s.cb_fcol[k] + 1;
     const int st = s.cb_stride[k];
     const int tot = st * nc;
-    const int tid = threadIdx.x, nt = blockDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int64_t *fbase = reinterpret_cast<int64_t *>(smem_raw);  // per blok: first target column, and its stride
+    int *fst = reinterpret_cast<int *>(fbase + PS_BLOKS);
+    T *inv = reinterpret_cast<T *>(fst + PS_BLOKS);
+    T *P = inv + 64;
+    T *Q = P + tot;
+    int *rb = reinterpret_cast<int *>(P + (FACT == FACT_GETRF ? 2 : 1) * tot);  // blok of each panel row
+    int *pair = rb + st;
     T *gL = L + s.cb_coef[k];
     T *gU = (FACT == FACT_GETRF) ? U + s.cb_coef[k] : nullptr;
-    T *Q = P + tot;
     batched_copy<8, T>(tot, [&](int i) { return gL[i]; }, [&](int i, T v) { P[i] = v; });
     if (FACT == FACT_GETRF) batched_copy<8, T>(tot, [&](int i) { return gU[i]; }, [&](int i, T v) { Q[i] = v; });
-    __shared__ int npiv;
-    if (tid == 0) npiv = 0;
+    const int fb = s.cb_fblok[k] + 1, B = s.cb_fblok[k + 1] - fb;  // off-diagonal bloks
     __syncthreads();
     if (FACT == FACT_GETRF) {  // L_kk += (U^T)_kk^T : the full diagonal block
-        for (int e = tid; e < nc * nc; e += nt) {
+        for (int e = tid; e < nc * nc; e += PS_THREADS) {
             int i = e % nc, j = e / nc;
             P[i + j * st] += Q[j + i * st];
         }
         __syncthreads();
     }
-    for (int c = 0; c < nc; c++) {
-        if (tid == 0) {
-            int np = npiv;
-            P[c + c * st] = static_pivot<T, FACT>(P[c + c * st], __ldg(fp.criterion), np);
-            npiv = np;
+    // U(k, c), k < c, of the diagonal block: L^T, D L^T (kept above the diagonal) or U
+    auto upper = [&](int kk, int c) -> T { return FACT == FACT_POTRF ? P[c + kk * st] : P[kk + c * st]; };
+    // Tables of bloks b0 .. b1 - 1: target base and stride, and for every later blok b2 the shift from
+    // a panel row of b2 to its row in the facing cblk of b.  pidx(b, b2): place of a pair.
+    auto pidx = [&](int b0, int b, int b2) { return (b - b0) * B - (b * (b - 1) - b0 * (b0 - 1)) / 2 + (b2 - b); };
+    auto shift_of = [&](int b, int b2) -> int {
+        const int f = s.bk_fcblk[fb + b], g = s.bk_frow[fb + b2];
+        int lo = s.cb_fblok[f], hi = s.cb_fblok[f + 1] - 1;
+        while (lo < hi) {  // last blok of f whose first row is <= g
+            const int mid = (lo + hi + 1) >> 1;
+            if (s.bk_frow[mid] <= g) lo = mid;
+            else hi = mid - 1;
         }
-        __syncthreads();
-        const T inv = T(1) / P[c + c * st];
-        for (int i = c + 1 + tid; i < st; i += nt) {
-            if (FACT == FACT_SYTRF && i < nc) P[c + i * st] = P[i + c * st];  // D*L^T into the upper part
-            P[i + c * st] *= inv;
+        return s.bk_rowoff[lo] + (g - s.bk_frow[lo]) - s.bk_rowoff[fb + b2];
+    };
+    auto tables = [&](int b0, int b1, int t, int nt) {
+        for (int b = b0 + t; b < b1; b += nt) {
+            const int f = s.bk_fcblk[fb + b], stf = s.cb_stride[f];
+            fbase[b - b0] = s.cb_coef[f] + (int64_t)(s.bk_frow[fb + b] - s.cb_fcol[f]) * stf;
+            fst[b - b0] = stf;
         }
-        __syncthreads();
-        const int w = nc - c - 1;
-        if (w > 0) {
-            const int h = st - c - 1;
-            for (int e = tid; e < h * w; e += nt) {
-                int i = c + 1 + e % h, j = c + 1 + e / h;
-                if (FACT == FACT_POTRF) {
-                    if (i >= j) P[i + j * st] -= P[i + c * st] * P[j + c * st];
-                } else if (FACT == FACT_SYTRF) {
-                    if (i >= j) P[i + j * st] -= P[i + c * st] * P[c + j * st];
-                } else {
-                    P[i + j * st] -= P[i + c * st] * P[c + j * st];
+        const int np = min(PS_PAIRS, pidx(b0, b1, b1));
+        for (int e = t; e < np; e += nt) {
+            int b = b0, r = e;
+            while (r >= B - b) r -= B - b++;
+            pair[e] = shift_of(b, b + r);
+        }
+    };
+    auto chunk_end = [&](int b0) {  // bloks whose tables fit, at least one
+        int b1 = b0 + 1;
+        while (b1 < B && b1 - b0 < PS_BLOKS && pidx(b0, b1 + 1, b1 + 1) <= PS_PAIRS) b1++;
+        return b1;
+    };
+    int npiv = 0;
+    if (warp == 0) {
+        const int i0 = min(lane, nc - 1), i1 = min(lane + 32, nc - 1);
+        for (int c = 0; c < nc; c++) {
+            T v0 = P[i0 + c * st], v1 = P[i1 + c * st];  // column c, rows lane and lane + 32
+#pragma unroll 4
+            for (int kk = 0; kk < c; kk++) {
+                const T u = upper(kk, c);
+                v0 -= P[i0 + kk * st] * u;
+                v1 -= P[i1 + kk * st] * u;
+            }
+            T w0 = T(0), w1 = T(0);  // GETRF: row c of U, columns lane and lane + 32
+            if (FACT == FACT_GETRF) {
+                w0 = P[c + i0 * st];
+                w1 = P[c + i1 * st];
+#pragma unroll 4
+                for (int kk = 0; kk < c; kk++) {
+                    const T l = P[c + kk * st];
+                    w0 -= l * P[kk + i0 * st];
+                    w1 -= l * P[kk + i1 * st];
                 }
             }
-            if (FACT == FACT_GETRF) {  // U^T rows below the diagonal block: A[j, r] -= L[j,c] U[c,r]
-                const int h2 = st - nc;
-                for (int e = tid; e < h2 * w; e += nt) {
-                    int r = nc + e % h2, j = c + 1 + e / h2;
-                    Q[r + j * st] -= P[j + c * st] * Q[r + c * st];
-                }
+            const T a = __shfl_sync(0xffffffffu, c < 32 ? v0 : v1, c & 31);
+            const T d = static_pivot<T, FACT>(a, __ldg(fp.criterion), npiv);
+            const T rd = T(1) / d;
+            __syncwarp();  // the reads of this step are done
+            if (lane == 0) {
+                P[c + c * st] = d;
+                inv[c] = rd;
+            }
+            if (lane > c && lane < nc) {
+                P[lane + c * st] = v0 * rd;
+                if (FACT == FACT_SYTRF) P[c + lane * st] = v0;
+                if (FACT == FACT_GETRF) P[c + lane * st] = w0;
+            }
+            if (lane + 32 > c && lane + 32 < nc) {
+                P[lane + 32 + c * st] = v1 * rd;
+                if (FACT == FACT_SYTRF) P[c + (lane + 32) * st] = v1;
+                if (FACT == FACT_GETRF) P[c + (lane + 32) * st] = w1;
+            }
+            __syncwarp();
+        }
+    } else {
+        for (int b = tid - 32; b < B; b += PS_THREADS - 32) {
+            const int r0 = s.bk_rowoff[fb + b], n = s.bk_lrow[fb + b] - s.bk_frow[fb + b] + 1;
+            for (int r = 0; r < n; r++) rb[r0 + r] = b;
+        }
+        if (B > 0) tables(0, chunk_end(0), tid - 32, PS_THREADS - 32);
+    }
+    __syncthreads();
+    // rows below the diagonal block, X U = A; GETRF: and the rows of U^T, X L^T = A (unit)
+    const int below = st - nc;
+    for (int e = tid; e < below * (FACT == FACT_GETRF ? 2 : 1); e += PS_THREADS) {
+        const bool us = FACT == FACT_GETRF && e >= below;
+        T *R = (us ? Q : P) + nc + (us ? e - below : e);
+        auto tri = [&](int kk, int c) -> T { return us ? P[c + kk * st] : upper(kk, c); };
+        for (int c0 = 0; c0 < nc; c0 += 4) {
+            const int c1 = min(c0 + 1, nc - 1), c2 = min(c0 + 2, nc - 1), c3 = min(c0 + 3, nc - 1);
+            T a0 = R[c0 * st], a1 = R[c1 * st], a2 = R[c2 * st], a3 = R[c3 * st];
+#pragma unroll 4
+            for (int kk = 0; kk < c0; kk++) {
+                const T x = R[kk * st];
+                a0 -= x * tri(kk, c0);
+                a1 -= x * tri(kk, c1);
+                a2 -= x * tri(kk, c2);
+                a3 -= x * tri(kk, c3);
+            }
+            if (!us) a0 *= inv[c0];
+            R[c0 * st] = a0;
+            if (c0 + 1 < nc) {
+                a1 -= a0 * tri(c0, c1);
+                if (!us) a1 *= inv[c1];
+                R[c1 * st] = a1;
+            }
+            if (c0 + 2 < nc) {
+                a2 = (a2 - a0 * tri(c0, c2)) - a1 * tri(c1, c2);
+                if (!us) a2 *= inv[c2];
+                R[c2 * st] = a2;
+            }
+            if (c0 + 3 < nc) {
+                a3 = ((a3 - a0 * tri(c0, c3)) - a1 * tri(c1, c3)) - a2 * tri(c2, c3);
+                if (!us) a3 *= inv[c3];
+                R[c3 * st] = a3;
             }
         }
-        __syncthreads();
     }
     if (FACT == FACT_GETRF) {  // (U^T)_kk = (L\U)_kk^T
-        for (int e = tid; e < nc * nc; e += nt) {
+        for (int e = tid; e < nc * nc; e += PS_THREADS) {
             int i = e % nc, j = e / nc;
             Q[j + i * st] = P[i + j * st];
         }
-        __syncthreads();
-        for (int i = tid; i < tot; i += nt) gU[i] = Q[i];
     }
-    for (int i = tid; i < tot; i += nt) gL[i] = P[i];
-    if (tid == 0 && npiv) atomicAdd(fp.nbpivots, npiv);
-    // the updates of every task of this cblk (core_zgemmsp_2d2d), from the
-    // factored panel still in shared memory, scattered into the facing panels
-    // with reductions; rtab / ctab: target rows and columns of one task
     __syncthreads();
-    int *rtab = reinterpret_cast<int *>(P + (FACT == FACT_GETRF ? 2 : 1) * tot);
-    int *ctab = rtab + st;
-    int *fbr = ctab + st;           // first rows of the facing cblk's bloks (when they fit)
-    int *fbo = fbr + PS_FB_CACHE;   // and their row offsets
-    const int *ridx = s.rowidx + s.cb_rowidx[k];
-    for (int b = s.cb_fblok[k] + 1; b < s.cb_fblok[k + 1]; b++) {
-        const int f = s.bk_fcblk[b];
-        const int row0 = s.bk_rowoff[b];
-        const int n = s.bk_lrow[b] - s.bk_frow[b] + 1;
-        const int M = st - row0;
-        const int fb0 = s.cb_fblok[f], nbf = s.cb_fblok[f + 1] - fb0;
-        const bool cached = nbf <= PS_FB_CACHE;
-        if (cached)
-            for (int e = tid; e < nbf; e += nt) {
-                fbr[e] = s.bk_frow[fb0 + e];
-                fbo[e] = s.bk_rowoff[fb0 + e];
-            }
-        __syncthreads();
-        for (int i = tid; i < M; i += nt) {
-            const int g = ridx[row0 + i];
-            int lo = 0, hi = nbf - 1;
-            while (lo < hi) {  // last blok of f whose first row is <= g
-                const int mid = (lo + hi + 1) >> 1;
-                if ((cached ? fbr[mid] : s.bk_frow[fb0 + mid]) <= g) lo = mid;
-                else hi = mid - 1;
-            }
-            rtab[i] = (cached ? fbo[lo] : s.bk_rowoff[fb0 + lo]) + (g - (cached ? fbr[lo] : s.bk_frow[fb0 + lo]));
+    for (int i = tid; i < tot; i += PS_THREADS) gL[i] = P[i];
+    if (FACT == FACT_GETRF)
+        for (int i = tid; i < tot; i += PS_THREADS) gU[i] = Q[i];
+    if (tid == 0 && npiv) atomicAdd(fp.nbpivots, npiv);
+    // updates, chunk by chunk of bloks
+    for (int b0 = 0; b0 < B;) {
+        const int b1 = chunk_end(b0);
+        if (b0 > 0) {
+            __syncthreads();
+            tables(b0, b1, tid, PS_THREADS);
+            __syncthreads();
         }
-        for (int j = tid; j < n; j += nt) ctab[j] = ridx[row0 + j] - s.cb_fcol[f];
-        __syncthreads();
-        T *Cl = L + s.cb_coef[f];
-        const int stf = s.cb_stride[f];
-        for (int e = tid; e < M * n; e += nt) {
-            const int i = e % M, j = e / M;
-            T v = T(0);
-            for (int c = 0; c < nc; c++) {
-                T bj = (FACT == FACT_GETRF) ? Q[(row0 + j) + c * st] : P[(row0 + j) + c * st];
-                if (FACT == FACT_SYTRF) bj *= P[c + c * st];
-                v += P[(row0 + i) + c * st] * bj;
-            }
-            atomicAdd(&Cl[rtab[i] + (size_t)ctab[j] * stf], -v);
+        for (int b = b0; b < b1; b++) {
+            const int row0 = s.bk_rowoff[fb + b], n = s.bk_lrow[fb + b] - s.bk_frow[fb + b] + 1;
+            const int nq = (n + 3) >> 2, stf = fst[b - b0];
+            const T *Bp = ((FACT == FACT_GETRF) ? Q : P) + row0;
+            auto update = [&](const T *Ap, const T *Bq, T *C, int skip) {
+                const int M = st - row0 - skip, items = M * nq;
+                // e / M by a multiplication, exact while e M < 2^32
+                const unsigned magic = 0xffffffffu / (unsigned)max(M, 1) + 1u;
+                const bool mul = M > 1 && (long long)items * M < (1LL << 32);
+                for (int e = (tid + 32 * b) & (PS_THREADS - 1); e < items; e += PS_THREADS) {
+                    const int jq = mul ? (int)__umulhi((unsigned)e, magic) : e / M;
+                    const int i = skip + e - jq * M, j = 4 * jq;
+                    const T *ap = Ap + row0 + i;
+                    const T *b0p = Bq + j, *b1p = Bq + min(j + 1, n - 1), *b2p = Bq + min(j + 2, n - 1),
+                            *b3p = Bq + min(j + 3, n - 1);
+                    T v0 = T(0), v1 = T(0), v2 = T(0), v3 = T(0);
+#pragma unroll 4
+                    for (int c = 0; c < nc; c++) {
+                        T a = ap[c * st];
+                        if (FACT == FACT_SYTRF) a *= P[c + c * st];
+                        v0 += a * b0p[c * st];
+                        v1 += a * b1p[c * st];
+                        v2 += a * b2p[c * st];
+                        v3 += a * b3p[c * st];
+                    }
+                    const int r = row0 + i, b2 = rb[r], px = pidx(b0, b, b2);
+                    T *dst = C + fbase[b - b0] + r + (px < PS_PAIRS ? pair[px] : shift_of(b, b2));
+                    atomicAdd(dst + (size_t)j * stf, -v0);
+                    if (j + 1 < n) atomicAdd(dst + (size_t)(j + 1) * stf, -v1);
+                    if (j + 2 < n) atomicAdd(dst + (size_t)(j + 2) * stf, -v2);
+                    if (j + 3 < n) atomicAdd(dst + (size_t)(j + 3) * stf, -v3);
+                }
+            };
+            update(P, Bp, L, 0);
+            // U side: rows strictly below the blok, into the U panel
+            if (FACT == FACT_GETRF) update(Q, P + row0, U, n);
         }
-        if (FACT == FACT_GETRF) {  // U side: rows strictly below the blok, into the U panel of f
-            T *Cu = U + s.cb_coef[f];
-            const int M1 = M - n;
-            for (int e = tid; e < M1 * n; e += nt) {
-                const int i = n + e % M1, j = e / M1;
-                T v = T(0);
-                for (int c = 0; c < nc; c++) v += Q[(row0 + i) + c * st] * P[(row0 + j) + c * st];
-                atomicAdd(&Cu[rtab[i] + (size_t)ctab[j] * stf], -v);
-            }
-        }
-        __syncthreads();
+        b0 = b1;
     }
 }
 
@@ -2858,7 +2947,7 @@ template <typename T, int FACT>
 void launch_panel_small(const DevStruct &s, const int *list, int count, size_t smem, T *L, T *U,
                         const FactParams &fp, cudaStream_t st) {
     if (count <= 0) return;
-    launch_k(k_panel_small<T, FACT>, count, 128, smem, st, s, list, L, U, fp);
+    launch_k(k_panel_small<T, FACT>, count, PS_THREADS, smem, st, s, list, L, U, fp);
 }
 
 // 16-CTA clusters of the LU kernel that the current device runs at once (0: none), for a
