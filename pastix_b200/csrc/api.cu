@@ -103,6 +103,9 @@ cudaError_t set_solve_attrs();
 void spmv_partition(int n, const int *rowptr, std::vector<int> &part);
 void launch_spmv_stream(int nblocks, const int *part, const int *rowptr, const int *col, const double *val,
                         double alpha, const double *x, double beta, double *y, cudaStream_t st);
+void launch_spmv_orig(int, const int *, const int *, const int *, const double *, const int *, double, const double *,
+                      double, double *, cudaStream_t);
+void launch_orig_index(int, int64_t, const int64_t *, const int *, int *, int *, cudaStream_t);
 void launch_spmv(int, int64_t, const int *, const int *, const double *, double, const double *, double, double *,
                  cudaStream_t);
 int reduce_partials();
@@ -236,6 +239,7 @@ struct Device {
     DBuf<double> vals, csr_val;
     DBuf<int64_t> lmap, umap, csr_src, perm;
     DBuf<int> csr_rowptr, csr_col, e_row, e_col;
+    DBuf<int> csr_colo, peri;  // columns in the caller's numbering, matrix row of every permuted row
     DBuf<int> spmv_part;     // row blocks of the streamed SpMV
     int spmv_nblocks = 0;
     // factor
@@ -1536,6 +1540,10 @@ static int device_setup(pastix_data_t *pd) {
     CUDA_TRY(d.e_col.upload(pd->e_col, st));
     std::vector<int64_t> perm(pd->order.permtab.begin(), pd->order.permtab.end());
     CUDA_TRY(d.perm.upload(perm, st));
+    CUDA_TRY(d.peri.alloc(pd->n));
+    CUDA_TRY(d.csr_colo.alloc(std::max<size_t>(1, pd->csr_col.size())));
+    pgpu::launch_orig_index((int)pd->n, (int64_t)pd->csr_col.size(), d.perm.p, d.csr_col.p, d.peri.p, d.csr_colo.p, st);
+    CUDA_TRY(cudaGetLastError());
     CUDA_TRY(d.vals.alloc(std::max<idx_t>(1, pd->nnz)));
     CUDA_TRY(d.csr_val.alloc(std::max<idx_t>(1, pd->csr_nnz)));
     CUDA_TRY(d.counters.alloc(4));
@@ -2882,10 +2890,19 @@ extern "C" int pgpu_spmv_device(pastix_data_t *pd, double alpha, const double *x
     if (!pd || !(pd->steps & STEP_CSC2BCSC) || !x || !y) return PASTIX_ERR_BADPARAMETER;
     Device &d = pd->dev;
     CUDA_TRY(cudaSetDevice(d.dev));
+    cudaStream_t st = (cudaStream_t)stream;  // the caller's stream; NULL = legacy default stream
+    if (x + pd->n <= y || y + pd->n <= x) {
+        launch_cls(pd, PC_SPMV, 1, [&] {
+            pgpu::launch_spmv_orig(d.spmv_nblocks, d.spmv_part.p, d.csr_rowptr.p, d.csr_colo.p, d.csr_val.p, d.peri.p,
+                                   alpha, x, beta, y, st);
+        }, st ? st : cudaStreamLegacy);
+        CUDA_TRY(cudaGetLastError());
+        return PASTIX_SUCCESS;
+    }
+    // y overlaps x: through permuted copies
     if (d.w1.n < (size_t)pd->n) CUDA_TRY(d.w1.alloc(pd->n));
     if (d.w2.n < (size_t)pd->n) CUDA_TRY(d.w2.alloc(pd->n));
     CUDA_TRY(cudaStreamSynchronize(d.stream));  // the work vectors are shared with the library stream
-    cudaStream_t st = (cudaStream_t)stream;     // the caller's stream; NULL = legacy default stream
     pgpu::launch_permute<double, double>((int)pd->n, 1, d.perm.p, 1, x, pd->n, d.w1.p, pd->n, st);
     pgpu::launch_permute<double, double>((int)pd->n, 1, d.perm.p, 1, y, pd->n, d.w2.p, pd->n, st);
     launch_cls(pd, PC_SPMV, 1, [&] {

@@ -43,9 +43,14 @@ __global__ void k_spmv(int n, const int *__restrict__ rowptr, const int *__restr
 // col into shared memory, then each thread sums one row of them.  A row longer
 // than SPMV_CAP gets a block of its own, reduced by the whole block.
 constexpr int SPMV_ROWS = 256, SPMV_CAP = 2304;
+// ORIG: x and y are in the numbering of the caller's matrix, col holds its
+// columns and peri the matrix row of each row of the CSR; otherwise both are
+// permuted and peri is not read.
+template <bool ORIG>
 __global__ void __launch_bounds__(256) k_spmv_stream(const int *__restrict__ part, const int *__restrict__ rowptr,
                                                      const int *__restrict__ col, const double *__restrict__ val,
-                                                     double alpha, const double *__restrict__ x, double beta,
+                                                     const int *__restrict__ peri, double alpha,
+                                                     const double *__restrict__ x, double beta,
                                                      double *__restrict__ y) {
     __shared__ double prod[SPMV_CAP];
     __shared__ double red[8];
@@ -61,7 +66,8 @@ __global__ void __launch_bounds__(256) k_spmv_stream(const int *__restrict__ par
             const int b = rowptr[r] - p0, e = rowptr[r + 1] - p0;
             double acc = 0.0;
             for (int q = b; q < e; q++) acc += prod[q];
-            y[r] = alpha * acc + (beta == 0.0 ? 0.0 : beta * y[r]);
+            const int o = ORIG ? peri[r] : r;
+            y[o] = alpha * acc + (beta == 0.0 ? 0.0 : beta * y[o]);
         }
     } else {  // one long row
         double acc = 0.0;
@@ -72,7 +78,8 @@ __global__ void __launch_bounds__(256) k_spmv_stream(const int *__restrict__ par
         if (tid == 0) {
             double t = 0.0;
             for (int w = 0; w < 8; w++) t += red[w];
-            y[r0] = alpha * t + (beta == 0.0 ? 0.0 : beta * y[r0]);
+            const int o = ORIG ? peri[r0] : r0;
+            y[o] = alpha * t + (beta == 0.0 ? 0.0 : beta * y[o]);
         }
     }
 }
@@ -326,7 +333,27 @@ void spmv_partition(int n, const int *rowptr, std::vector<int> &part) {
 }
 void launch_spmv_stream(int nblocks, const int *part, const int *rowptr, const int *col, const double *val,
                         double alpha, const double *x, double beta, double *y, cudaStream_t st) {
-    if (nblocks > 0) k_spmv_stream<<<nblocks, 256, 0, st>>>(part, rowptr, col, val, alpha, x, beta, y);
+    if (nblocks > 0) k_spmv_stream<false><<<nblocks, 256, 0, st>>>(part, rowptr, col, val, nullptr, alpha, x, beta, y);
+}
+// The same with x and y (distinct) in the caller's numbering.  Moving x and y to
+// the permuted numbering and y back took three more passes and launches: a
+// residual of the 80^3 Laplacian 37 -> 28 us (B200), although the kernel itself,
+// with less local columns, takes 21 us instead of 13.
+void launch_spmv_orig(int nblocks, const int *part, const int *rowptr, const int *colo, const double *val,
+                      const int *peri, double alpha, const double *x, double beta, double *y, cudaStream_t st) {
+    if (nblocks > 0) k_spmv_stream<true><<<nblocks, 256, 0, st>>>(part, rowptr, colo, val, peri, alpha, x, beta, y);
+}
+// peri[perm[i]] = i, then colo[p] = peri[col[p]]
+__global__ void k_peri(int n, const int64_t *__restrict__ perm, int *__restrict__ peri) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) peri[perm[i]] = i;
+}
+__global__ void k_colo(int64_t nnz, const int *__restrict__ col, const int *__restrict__ peri, int *__restrict__ colo) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (int64_t)gridDim.x * blockDim.x)
+        colo[p] = peri[col[p]];
+}
+void launch_orig_index(int n, int64_t nnz, const int64_t *perm, const int *col, int *peri, int *colo, cudaStream_t st) {
+    k_peri<<<(int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8)), 256, 0, st>>>(n, perm, peri);
+    if (nnz > 0) k_colo<<<(int)std::min<int64_t>((nnz + 255) / 256, 148 * 16), 256, 0, st>>>(nnz, col, peri, colo);
 }
 
 void launch_spmv(int n, int64_t nnz, const int *rowptr, const int *col, const double *val, double alpha,
