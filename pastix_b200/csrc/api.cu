@@ -98,6 +98,7 @@ void launch_update_i8(const DevStruct &, const UpdTile *, int, double *, double 
 cudaError_t set_i8_attrs();
 int sm_count();
 int solve_rows_per_tile();
+bool solve_fuse_rows(int count, int nrhs);
 cudaError_t set_solve_attrs();
 // vec.cu
 void spmv_partition(int n, const int *rowptr, std::vector<int> &part);
@@ -199,7 +200,7 @@ struct LevelLists {
     int tr32_0, tr32_1;     // FP32: DMMA TRSM tiles of the wide cblks the GEMM form does not take
     int ti_maxnzb;          // 32-column blocks of the widest cblk with a triangular inverse
     int cb0, cb1;           // all cblks of the level (solve diag)
-    int st0, st1;           // solve row tiles
+    int st0, stw, st1;      // solve row tiles: of the wide cblks, then of the narrow ones
     int maxnc;
     int trsm_maxnc;         // widest cblk with TRSM tiles
     int diag_maxnc;         // widest cblk of the large list
@@ -1231,6 +1232,12 @@ static int build_maps_and_lists(pastix_data_t *pd) {
                 if (st > nc) L.trsm_smem_elems = std::max<size_t>(L.trsm_smem_elems, (size_t)pgpu::trsm_smem_elems((int)nc));
                 if (st > nc) L.trsm_maxnc = std::max<int>(L.trsm_maxnc, (int)nc);
             }
+            if (st * nc > SMALL_PANEL_ELEMS)
+                for (idx_t r = nc; r < st; r += SR) pd->solve_tiles.push_back(pgpu::RowTile{(int)k, (int)r});
+        }
+        L.stw = (int)pd->solve_tiles.size();
+        for (int q = L.small0; q < (int)pd->small_list.size(); q++) {
+            const idx_t k = pd->small_list[q], nc = sv.cb_lcol[k] - sv.cb_fcol[k] + 1, st = sv.cb_stride[k];
             for (idx_t r = nc; r < st; r += SR) pd->solve_tiles.push_back(pgpu::RowTile{(int)k, (int)r});
         }
         L.spl0 = (int)pd->split_slabs.size();
@@ -1990,9 +1997,10 @@ static void sweep_forward(pastix_data_t *pd, const T *P, int unit, int zside, in
                                          zside, scaled, Ld, Y, ldy, nrhs, tinv_of<T>(d), d.ti_off.p, lv.ntinv,
                                          d.stream);
         });
-        launch_cls(pd, PC_FWD_UPDATE, lv.st1 - lv.st0, [&] {
-            pgpu::launch_fwd_update<T>(d.ds, d.solve_tiles.p + lv.st0, lv.st1 - lv.st0, lv.maxnc, P, Y, ldy, nrhs,
-                                       d.stream);
+        // without the rows that the narrow cblks' diagonal kernel has applied
+        const int nt = (pgpu::solve_fuse_rows(lv.small1 - lv.small0, nrhs) ? lv.stw : lv.st1) - lv.st0;
+        launch_cls(pd, PC_FWD_UPDATE, nt, [&] {
+            pgpu::launch_fwd_update<T>(d.ds, d.solve_tiles.p + lv.st0, nt, lv.maxnc, P, Y, ldy, nrhs, d.stream);
         });
     }
 }
@@ -2004,9 +2012,9 @@ static void sweep_backward(pastix_data_t *pd, const T *P, int unit, int zside, i
     const T *Dinv = reinterpret_cast<const T *>(d.dinv.p);
     for (size_t l = pd->levels.size(); l-- > 0;) {
         const LevelLists &lv = pd->levels[l];
-        launch_cls(pd, PC_BWD_UPDATE, lv.st1 - lv.st0, [&] {
-            pgpu::launch_bwd_update<T>(d.ds, d.solve_tiles.p + lv.st0, lv.st1 - lv.st0, lv.maxnc, P, Y, ldy, nrhs,
-                                       d.stream);
+        const int nt = (pgpu::solve_fuse_rows(lv.small1 - lv.small0, nrhs) ? lv.stw : lv.st1) - lv.st0;
+        launch_cls(pd, PC_BWD_UPDATE, nt, [&] {
+            pgpu::launch_bwd_update<T>(d.ds, d.solve_tiles.p + lv.st0, nt, lv.maxnc, P, Y, ldy, nrhs, d.stream);
         });
         launch_cls(pd, PC_BWD_DIAG, lv.small1 - lv.small0, [&] {
             pgpu::launch_bwd_diag<T>(d.ds, d.small_list.p + lv.small0, lv.small1 - lv.small0, lv.maxnc, P, unit, Y,

@@ -147,7 +147,11 @@ __global__ void __launch_bounds__(256) k_bwd_diag(DevStruct s, const int *__rest
 // One right-hand side: one warp per narrow cblk (width <= 64, since
 // stride * width <= 4096), eight cblks per CTA -- the leaves of the tree are
 // tens of thousands of such cblks, and a CTA each left seven of its warps
-// idle.  y_k lives in two registers per lane (columns lane, 32 + lane); the
+// idle.  In levels of many narrow cblks (solve_fuse_rows) the warp also applies
+// the rows below its diagonal block: as 64 x 64 update tiles a leaf of ten
+// columns kept a sixth of a CTA's threads busy, and the backward sums went
+// through atomics.  Lower four levels of the 100^3 Laplacian, FP32 factors,
+// forward: 324 -> 100 us (B200).  y_k lives in two registers per lane (columns lane, 32 + lane); the
 // substitution steps are those of k_fwd_diag / k_bwd_diag.
 //
 // The 32 x 32 block that the sweep starts with is loaded ahead of pdl_wait: it
@@ -189,9 +193,25 @@ __device__ __forceinline__ T warp_bwd_block(const T (&d)[32], T rd, int nb, int 
     return v;
 }
 
+// Sum over the 32 lanes of v[u] for every u at once (butterfly transpose
+// reduction, 31 shuffles): on return lane l holds in v[0] the sum of v[l].
 template <typename T>
-__global__ void __launch_bounds__(256) k_fwd_diag_w(DevStruct s, const int *__restrict__ list, int count, const T *P,
-                                                     int unit, T *Y) {
+__device__ __forceinline__ void lane_sums32(T (&v)[32], int lane) {
+#pragma unroll
+    for (int sft = 16; sft >= 1; sft >>= 1) {
+        const bool upper = (lane & sft) != 0;
+#pragma unroll
+        for (int u = 0; u < sft; u++) {
+            const T send = upper ? v[u] : v[u + sft];
+            const T keep = upper ? v[u + sft] : v[u];
+            v[u] = keep + __shfl_xor_sync(0xffffffffu, send, sft);
+        }
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_fwd_diag_w(DevStruct s, const int *__restrict__ list, int count, const T *P,
+                                                     int unit, T *Y, int rows) {
     pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int w = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -220,11 +240,34 @@ __global__ void __launch_bounds__(256) k_fwd_diag_w(DevStruct s, const int *__re
     }
     if (lane < nc) Y[fc + lane] = y0;
     if (32 + lane < nc) Y[fc + 32 + lane] = y1;
+    if (!rows) return;
+    // y[row(r)] -= P[r, :] y_k, two rows per lane, eight columns' loads in flight
+    const int *ridx = s.rowidx + s.cb_rowidx[k];
+    for (int r0 = nc; r0 < st; r0 += 64) {
+        const int ra = r0 + lane, rb = ra + 32;
+        T acc0 = T(0), acc1 = T(0);
+        for (int c0 = 0; c0 < nc; c0 += 8) {
+            T p0[8], p1[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                p0[u] = (ra < st && c0 + u < nc) ? D[ra + (size_t)(c0 + u) * st] : T(0);
+                p1[u] = (rb < st && c0 + u < nc) ? D[rb + (size_t)(c0 + u) * st] : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const T yc = __shfl_sync(0xffffffffu, c0 < 32 ? y0 : y1, (c0 + u) & 31);
+                acc0 += p0[u] * yc;
+                acc1 += p1[u] * yc;
+            }
+        }
+        if (ra < st) atomicAdd(&Y[ridx[ra]], -acc0);
+        if (rb < st) atomicAdd(&Y[ridx[rb]], -acc1);
+    }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_bwd_diag_w(DevStruct s, const int *__restrict__ list, int count, const T *P,
-                                                     int unit, T *Y) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_bwd_diag_w(DevStruct s, const int *__restrict__ list, int count, const T *P,
+                                                     int unit, T *Y, int rows) {
     pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int w = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -236,10 +279,27 @@ __global__ void __launch_bounds__(256) k_bwd_diag_w(DevStruct s, const int *__re
     const T *D = P + s.cb_coef[k];
     T d[32], rd;
     const int jl = nc > 32 ? 32 : 0;  // the last block goes first
-    warp_bwd_load<T>(D, st, jl, nc - jl, unit, lane, d, rd);
+    const int *ridx = s.rowidx + s.cb_rowidx[k];
+    if (!rows) warp_bwd_load<T>(D, st, jl, nc - jl, unit, lane, d, rd);
     pdl_wait();
     T y0 = lane < nc ? Y[fc + lane] : T(0);
     T y1 = 32 + lane < nc ? Y[fc + 32 + lane] : T(0);
+    // x_k -= P_off^T x[rows]: lanes over the rows, the 32 column sums by one butterfly
+    for (int cb = jl; rows && cb >= 0; cb -= 32) {
+        T v[32];
+#pragma unroll
+        for (int u = 0; u < 32; u++) v[u] = T(0);
+        for (int r = nc + lane; r < st; r += 32) {
+            const T xr = Y[ridx[r]];
+#pragma unroll
+            for (int u = 0; u < 32; u++)
+                if (cb + u < nc) v[u] += D[r + (size_t)(cb + u) * st] * xr;
+        }
+        lane_sums32(v, lane);
+        if (cb) y1 -= v[0];
+        else y0 -= v[0];
+    }
+    if (rows) warp_bwd_load<T>(D, st, jl, nc - jl, unit, lane, d, rd);
     if (nc > 32) {  // the last block first, then its contribution to rows 0..31: y0 -= D[32 + c, lane] y1[c]
         y1 = warp_bwd_block<T>(d, rd, nc - 32, lane, y1);
         T acc = T(0);
@@ -465,21 +525,6 @@ __global__ void __cluster_dims__(TC, 1, 1) __launch_bounds__(256)
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
                 if (lane == 0 && c0 + u < nc && j < nr) Y[fc + c0 + u + (size_t)(j0 + j) * ldy] = (T)v;
             }
-    }
-}
-
-// Sum over the 32 lanes of v[u] for every u at once (butterfly transpose
-// reduction, 31 shuffles): on return lane l holds in v[0] the sum of v[l].
-__device__ __forceinline__ void lane_sums32(float (&v)[32], int lane) {
-#pragma unroll
-    for (int sft = 16; sft >= 1; sft >>= 1) {
-        const bool upper = (lane & sft) != 0;
-#pragma unroll
-        for (int u = 0; u < sft; u++) {
-            const float send = upper ? v[u] : v[u + sft];
-            const float keep = upper ? v[u + sft] : v[u];
-            v[u] = keep + __shfl_xor_sync(0xffffffffu, send, sft);
-        }
     }
 }
 
@@ -919,13 +964,20 @@ __global__ void k_diag_scale(DevStruct s, const T *L, T *Y, int ldy, int nrhs) {
 }
 
 // ------------------------------ launchers ---------------------------------
+// Whether the diagonal kernels of a level's `count` narrow cblks apply their rows
+// too: one right-hand side, and enough cblks that a warp each fills the SMs.
+// Levels of few, larger cblks take longer that way than two launches (512^2
+// diffusion, FP64: 64 cblks 26 us forward and 28 backward against about 10; 2048
+// and more 11 and 25 against 20 and 30).
+bool solve_fuse_rows(int count, int nrhs) { return nrhs == 1 && count >= 1024; }
 // One right-hand side or groups of 8 (a group's missing columns are masked).
 template <typename T>
 void launch_fwd_diag(const DevStruct &s, const int *list, int count, int maxnc, const T *P, int unit, T *Y, int ldy,
                      int nrhs, cudaStream_t st) {
     if (count <= 0) return;
     if (nrhs == 1)  // narrow cblks (width <= 64): one warp each
-        launch_k(k_fwd_diag_w<T>, dim3((count + 7) / 8), dim3(256), 0, st, s, list, count, P, unit, Y);
+        launch_k(k_fwd_diag_w<T>, dim3((count + 7) / 8), dim3(256), 0, st, s, list, count, P, unit, Y,
+                 (int)solve_fuse_rows(count, nrhs));
     else
         launch_k(k_fwd_diag<T, 8>, dim3(count, (nrhs + 7) / 8), dim3(256), 8 * (size_t)maxnc * sizeof(T), st, s, list, P,
                  unit, Y, ldy, nrhs);
@@ -935,7 +987,8 @@ void launch_bwd_diag(const DevStruct &s, const int *list, int count, int maxnc, 
                      int nrhs, cudaStream_t st) {
     if (count <= 0) return;
     if (nrhs == 1)
-        launch_k(k_bwd_diag_w<T>, dim3((count + 7) / 8), dim3(256), 0, st, s, list, count, P, unit, Y);
+        launch_k(k_bwd_diag_w<T>, dim3((count + 7) / 8), dim3(256), 0, st, s, list, count, P, unit, Y,
+                 (int)solve_fuse_rows(count, nrhs));
     else
         launch_k(k_bwd_diag<T, 8>, dim3(count, (nrhs + 7) / 8), dim3(256), 8 * (size_t)maxnc * sizeof(T), st, s, list, P,
                  unit, Y, ldy, nrhs);
