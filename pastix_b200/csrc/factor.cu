@@ -2160,6 +2160,20 @@ __global__ void __cluster_dims__(DC, 1, 1) __launch_bounds__(256, 1)
         dg_copy<8>(
             nc - lop, nb, [&](int r, int c) { return W[r * DG_LD + c]; },
             [&](int r, int c, double v) { A[(lop + r) + (size_t)(32 * p + c) * st] = (T)v; });
+        // the panel's part of the other triangle, from shared memory too, so that
+        // no CTA walks the whole block at the end (by one CTA the copies took 50 to
+        // 100 us of the 300 to 400 of a 300-column LDL^T or LU block)
+        if (FACT == FACT_SYTRF) {  // above the diagonal: D L^T
+            __syncthreads();       // the diagonal block's upper part was written above
+            for (int r = warp; r < nc - lop; r += 8)
+                if (lane < nb && lane < r)
+                    A[(32 * p + lane) + (size_t)(lop + r) * st] = (T)W[lane * DG_LD + lane] * (T)W[r * DG_LD + lane];
+        }
+        if (FACT == FACT_GETRF) {  // (U^T)_kk = (L\U)_kk^T
+            T *Ut = U + s.cb_coef[k];
+            for (int r = warp; r < nc; r += 8)
+                if (lane < nb) Ut[(32 * p + lane) + (size_t)r * st] = (T)W[r * DG_LD + lane];
+        }
     };
     constexpr int DC_FOLLOW = 6;
     auto factor_panel = [&](int q, int pu) {
@@ -2251,25 +2265,7 @@ __global__ void __cluster_dims__(DC, 1, 1) __launch_bounds__(256, 1)
     // GETRF: this CTA's panels are final: write them out
     if (FACT == FACT_GETRF)
         for (int p = rank; p < np; p += DC) write_panel(p);
-    __threadfence();
-    cluster.sync();  // all panels written; no CTA leaves while its shared memory may still be read
-    if (rank == 0) {
-        if (FACT == FACT_SYTRF) {  // upper part of the diagonal block holds D L^T
-            batched_copy<8, T>(
-                nc * nc,
-                [&](int e) {
-                    int i = e % nc, j = e / nc;
-                    return (i < j) ? A[i + (size_t)i * st] * A[j + (size_t)i * st] : T(0);
-                },
-                [&](int e, T v) { int i = e % nc, j = e / nc; if (i < j) A[i + (size_t)j * st] = v; });
-        }
-        if (FACT == FACT_GETRF) {  // (U^T)_kk = (L\U)_kk^T
-            T *Ut = U + s.cb_coef[k];
-            batched_copy<8, T>(
-                nc * nc, [&](int e) { int i = e % nc, j = e / nc; return A[i + (size_t)j * st]; },
-                [&](int e, T v) { int i = e % nc, j = e / nc; Ut[j + (size_t)i * st] = v; });
-        }
-    }
+    cluster.sync();  // no CTA leaves while its shared memory may still be read
     __syncthreads();
     if (tid == 0 && npiv) atomicAdd(fp.nbpivots, npiv);
 }
