@@ -215,6 +215,7 @@ struct Device {
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;                      // FP32 factorization: updates of later levels
     std::vector<cudaEvent_t> ev_chain, ev_rest;       // per level: panels final / far updates done
+    cudaEvent_t ev_fact[2] = {nullptr, nullptr};      // around a factorization (DPARM_FACT_TIME)
     // structure
     DBuf<int> cb_fcol, cb_lcol, cb_stride, cb_fblok, bk_frow, bk_lrow, bk_rowoff, bk_fcblk, rowidx;
     DBuf<int64_t> cb_coef, cb_rowidx, cb_dinv, sp_off;
@@ -250,7 +251,7 @@ struct Device {
     DBuf<int> counters;      // [0] nbpivots, [1] status
     DBuf<int> queues;        // tile work-queue heads of the tcgen05 launches, 3 per level, zeroed per factorization
     DBuf<double> dcscr;      // finished panels of the cluster diagonal kernel (read by the cluster's other CTAs)
-    DBuf<double> crit;       // static pivoting threshold of the current factorization
+    DBuf<double> crit;       // [0] static pivoting threshold of the current factorization, [1] ||A||_F
     DBuf<double> part, scal; // reduction partials, scalars
     DBuf<double> w1, w2;     // permuted double work vectors
     DBuf<float> wf;          // float work for mixed precision
@@ -329,7 +330,6 @@ struct pastix_data_s {
     int factotype = PastixFactPOTRF;
     int mixed = 0;
     double anorm = 0.0;
-    double crit_host = 0.0;  // source of the threshold's copy to the device
     // bucket boundaries of the update tiles (pgpu_set_tuning / pgpu_autotune):
     // FP64 tasks with blok height >= tune_dmma_n and source width >= tune_dmma_k take
     // 128 x 64 DMMA tiles, the others 64 x 64 SIMT tiles; FP32 tasks whose source is
@@ -559,6 +559,8 @@ extern "C" void pastixFinalize(pastix_data_t **pd) {
         if (p->dev.side) cudaStreamSynchronize(p->dev.side);
         for (auto *v : {&p->dev.ev_chain, &p->dev.ev_rest})
             for (cudaEvent_t e : *v) cudaEventDestroy(e);
+        for (cudaEvent_t e : p->dev.ev_fact)
+            if (e) cudaEventDestroy(e);
         if (p->dev.side) cudaStreamDestroy(p->dev.side);
     }
     delete p;  // DBuf destructors free device memory
@@ -1488,6 +1490,8 @@ static int device_setup(pastix_data_t *pd) {
     CUDA_TRY(cudaSetDevice(d.dev));
     if (!d.stream) CUDA_TRY(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
     if (!d.side) CUDA_TRY(cudaStreamCreateWithFlags(&d.side, cudaStreamNonBlocking));
+    for (auto &e : d.ev_fact)
+        if (!e) CUDA_TRY(cudaEventCreate(&e));
     while (d.ev_chain.size() < pd->levels.size()) {
         cudaEvent_t a, b;
         CUDA_TRY(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
@@ -1556,7 +1560,7 @@ static int device_setup(pastix_data_t *pd) {
     CUDA_TRY(d.counters.alloc(4));
     CUDA_TRY(d.queues.alloc(std::max<size_t>(1, 3 * pd->levels.size())));
     CUDA_TRY(d.dcscr.alloc(pgpu::diag_cluster_scratch_doubles()));
-    CUDA_TRY(d.crit.alloc(1));
+    CUDA_TRY(d.crit.alloc(2));
     CUDA_TRY(cudaMemsetAsync(d.counters.p, 0, 4 * sizeof(int), st));
     CUDA_TRY(d.part.alloc(pgpu::reduce_partials()));
     CUDA_TRY(d.scal.alloc(64));
@@ -1598,13 +1602,12 @@ struct PdlScope {
 // numerical factorization
 // ---------------------------------------------------------------------------
 template <typename T, int F>
-static int run_factor(pastix_data_t *pd, double criterion) {
+static int run_factor(pastix_data_t *pd) {
     Device &d = pd->dev;
     cudaStream_t st = d.stream;
     T *L = reinterpret_cast<T *>(d.Lc.p);
     T *U = reinterpret_cast<T *>(d.Uc.p);
     T *Dinv = reinterpret_cast<T *>(d.dinv.p);
-    (void)criterion;  // copied to d.crit by the caller
     pgpu::FactParams fp{d.crit.p, d.counters.p, d.counters.p + 1, d.dcscr.p};
     // FP32: the updates of level l whose targets sit two or more levels up run on a
     // second stream and overlap level l + 1 (all FP32 update writes are reductions)
@@ -1755,17 +1758,26 @@ __global__ void k_gather_csr(int64_t nnz, const int64_t *__restrict__ src, const
         out[q] = vals[src[q]];
 }
 
-// bcsc analogue: permuted CSR values + ||A||_F (sopalin/pastix_task_sopalin.c:93-160)
+// Static pivoting threshold (sopalin/pastix_task_sopalin.c:464-495) from the norm
+// crit[1] = ||A||_F: crit[0] = scale * (relative ? ||A||_F : 1)
+__global__ void k_threshold(double *crit, double scale, int relative) { crit[0] = relative ? scale * crit[1] : scale; }
+
+static int fetch_norm(pastix_data_t *pd) {
+    double nrm = 0;
+    CUDA_TRY(cudaMemcpyAsync(&nrm, pd->dev.crit.p + 1, sizeof(double), cudaMemcpyDeviceToHost, pd->dev.stream));
+    CUDA_TRY(cudaStreamSynchronize(pd->dev.stream));
+    pd->anorm = nrm;
+    pd->dparm[DPARM_A_NORM] = nrm;
+    return PASTIX_SUCCESS;
+}
+
+// bcsc analogue: permuted CSR values + ||A||_F (sopalin/pastix_task_sopalin.c:93-160); the norm stays on the device
 static int values_to_csr(pastix_data_t *pd) {
     Device &d = pd->dev;
     int blocks = (int)std::min<int64_t>((pd->csr_nnz + 255) / 256, 148 * 16);
     k_gather_csr<<<std::max(blocks, 1), 256, 0, d.stream>>>(pd->csr_nnz, d.csr_src.p, d.vals.p, d.csr_val.p);
-    pgpu::launch_dot(pd->csr_nnz, d.csr_val.p, d.csr_val.p, d.part.p, 1, d.scal.p, d.stream);
-    double nrm = 0;
-    CUDA_TRY(cudaMemcpyAsync(&nrm, d.scal.p, sizeof(double), cudaMemcpyDeviceToHost, d.stream));
-    CUDA_TRY(cudaStreamSynchronize(d.stream));
-    pd->anorm = nrm;
-    pd->dparm[DPARM_A_NORM] = nrm;
+    pgpu::launch_dot(pd->csr_nnz, d.csr_val.p, d.csr_val.p, d.part.p, 1, d.crit.p + 1, d.stream);
+    CUDA_TRY(cudaGetLastError());
     return PASTIX_SUCCESS;
 }
 
@@ -1785,7 +1797,7 @@ static int spm2bcsc_common(pastix_data_t *pd, const void *values, bool on_device
     return PASTIX_SUCCESS;
 }
 
-extern "C" int pastix_subtask_spm2bcsc(pastix_data_t *pd, spmatrix_t *spm) {
+static int spm2bcsc_host(pastix_data_t *pd, spmatrix_t *spm) {
     if (!pd) return PASTIX_ERR_BADPARAMETER;
     int rc = check_spm(spm);
     if (rc) return rc;
@@ -1795,6 +1807,11 @@ extern "C" int pastix_subtask_spm2bcsc(pastix_data_t *pd, spmatrix_t *spm) {
     }
     if (!spm->values) return PASTIX_ERR_BADPARAMETER;
     return spm2bcsc_common(pd, spm->values, false, spm->flttype);
+}
+
+extern "C" int pastix_subtask_spm2bcsc(pastix_data_t *pd, spmatrix_t *spm) {
+    int rc = spm2bcsc_host(pd, spm);
+    return rc ? rc : fetch_norm(pd);
 }
 
 // coeftabInit (sopalin/coeftab.c:205): allocate and fill the panels
@@ -1884,39 +1901,39 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
     Device &d = pd->dev;
     CUDA_TRY(cudaSetDevice(d.dev));
     double *dparm = pd->dparm;
-    double threshold;
-    if (dparm[DPARM_EPSILON_MAGN_CTRL] < 0.) threshold = -dparm[DPARM_EPSILON_MAGN_CTRL];
-    else if (dparm[DPARM_EPSILON_MAGN_CTRL] == 0.) threshold = ldexp(1.0, -53) * pd->anorm;  // dlamch('e') * ||A||
-    else threshold = dparm[DPARM_EPSILON_MAGN_CTRL] * pd->anorm;
+    // dlamch('e') * ||A|| by default, |magnitude control| when negative, else relative to ||A||
+    const double magn = dparm[DPARM_EPSILON_MAGN_CTRL];
+    k_threshold<<<1, 1, 0, d.stream>>>(d.crit.p, magn < 0. ? -magn : (magn == 0. ? ldexp(1.0, -53) : magn), magn >= 0.);
     CUDA_TRY(cudaMemsetAsync(d.counters.p, 0, 2 * sizeof(int), d.stream));
-    pd->crit_host = threshold;
-    CUDA_TRY(cudaMemcpyAsync(d.crit.p, &pd->crit_host, sizeof(double), cudaMemcpyHostToDevice, d.stream));
-    CUDA_TRY(cudaStreamSynchronize(d.stream));
-    double t0 = now_s();
+    CUDA_TRY(cudaEventRecord(d.ev_fact[0], d.stream));
     int fk = fact_kind(pd), rc;
     if (pd->mixed) {
         // FP32 factors: launched kernel by kernel.  Replayed as a graph, the same launches ran
         // 12% slower on a B200 (100^3 Laplacian: 83 ms against 74 ms, with or without the side
         // stream in the graph), so only the solves of this precision are graphed.
-        if (fk == pgpu::FACT_POTRF) rc = run_factor<float, pgpu::FACT_POTRF>(pd, threshold);
-        else if (fk == pgpu::FACT_SYTRF) rc = run_factor<float, pgpu::FACT_SYTRF>(pd, threshold);
-        else rc = run_factor<float, pgpu::FACT_GETRF>(pd, threshold);
+        if (fk == pgpu::FACT_POTRF) rc = run_factor<float, pgpu::FACT_POTRF>(pd);
+        else if (fk == pgpu::FACT_SYTRF) rc = run_factor<float, pgpu::FACT_SYTRF>(pd);
+        else rc = run_factor<float, pgpu::FACT_GETRF>(pd);
     } else {
         // FP64: the whole level sequence is one CUDA graph per (kind, buffers)
         const std::vector<uintptr_t> key{1, (uintptr_t)fk, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p,
                                          (uintptr_t)d.i8_img0.p, (uintptr_t)d.i8_img1.p, (uintptr_t)d.i8_sc0.p,
                                          (uintptr_t)d.i8_sc1.p};
         rc = run_graphed(pd, key, [&]() -> int {
-            if (fk == pgpu::FACT_POTRF) return run_factor<double, pgpu::FACT_POTRF>(pd, threshold);
-            if (fk == pgpu::FACT_SYTRF) return run_factor<double, pgpu::FACT_SYTRF>(pd, threshold);
-            return run_factor<double, pgpu::FACT_GETRF>(pd, threshold);
+            if (fk == pgpu::FACT_POTRF) return run_factor<double, pgpu::FACT_POTRF>(pd);
+            if (fk == pgpu::FACT_SYTRF) return run_factor<double, pgpu::FACT_SYTRF>(pd);
+            return run_factor<double, pgpu::FACT_GETRF>(pd);
         });
     }
     if (rc) return rc;
     int cnt[2] = {0, 0};
+    CUDA_TRY(cudaEventRecord(d.ev_fact[1], d.stream));
     CUDA_TRY(cudaMemcpyAsync(cnt, d.counters.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, d.stream));
-    CUDA_TRY(cudaStreamSynchronize(d.stream));
-    double t = now_s() - t0;
+    rc = fetch_norm(pd);
+    if (rc) return rc;
+    float ms = 0;
+    CUDA_TRY(cudaEventElapsedTime(&ms, d.ev_fact[0], d.ev_fact[1]));
+    const double t = ms * 1e-3;
     if (cnt[1] != 0) { perr("device status %d after factorization", cnt[1]); return PASTIX_ERR_INTERNAL; }
     dparm[DPARM_FACT_TIME] = t;
     dparm[DPARM_FACT_FLOPS] = t > 0 ? dparm[DPARM_FACT_THFLOPS] / t : 0.0;
@@ -1927,8 +1944,7 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
 }
 
 extern "C" int pastix_task_numfact(pastix_data_t *pd, spmatrix_t *spm) {
-    if (!pd) return PASTIX_ERR_BADPARAMETER;
-    int rc = pastix_subtask_spm2bcsc(pd, spm);
+    int rc = spm2bcsc_host(pd, spm);
     if (rc) return rc;
     rc = pastix_subtask_bcsc2ctab(pd);
     if (rc) return rc;
