@@ -93,7 +93,7 @@ void launch_split_i8(const DevStruct &, const SplitSlab *, int, const double *, 
                      unsigned char *, double *, int, cudaStream_t);
 template <int F>
 void launch_update_i8(const DevStruct &, const UpdTile *, int, double *, double *, const unsigned char *,
-                      const unsigned char *, const double *, const double *, const int64_t *, int *, int *, int,
+                      const unsigned char *, const double *, const double *, const int64_t *, int *, int *, bool,
                       cudaStream_t);
 cudaError_t set_i8_attrs();
 int sm_count();
@@ -191,7 +191,7 @@ struct LevelLists {
     int updb0, updb1;       // big update tiles (128 x 64): DMMA for FP64
     int updt0, updt1;       // the same tasks in 128-row aligned windows: tcgen05 for FP32
     int updm, updbm;        // FP64 lists: tiles from here on belong to tasks that the integer kernel takes
-    int upi0, upi1;         // those tasks in 128 x 128 windows: integer slices on tcgen05 (FP64 factors)
+    int upi0, upin, upi1;   // those tasks in 128 x 128 windows (integer slices on tcgen05, FP64 factors): next level's targets, later ones
     int isl0, isl1;         // 128-row slabs of their source cblks, cut into digits
     int updtn, updsn;       // FP32 lists: tiles before these target the next level's cblks
     int spl0, spl1;         // 128-row slabs of the level's cblks split into BF16 terms (FP32)
@@ -315,7 +315,7 @@ struct pastix_data_s {
     std::vector<pgpu::UpdTile> upd_tiles, upd_big_tiles, upd_tc_tiles, upd_tiles32, upd_i8_tiles;
     std::vector<pgpu::SplitSlab> i8_slabs;
     std::vector<int64_t> i8_off;             // byte offset of each cblk's digit image in its level's images (-1: none)
-    int64_t i8_total = 0;                    // bytes of the largest level's images
+    int64_t i8_total = 0;                    // bytes of the largest level's images (two areas of this size)
     std::vector<pgpu::TaskDev> tasks;
     std::vector<int64_t> cb_dinv;
     std::vector<int64_t> sp_off;             // byte offset of each cblk's BF16 image (-1: none)
@@ -1288,6 +1288,7 @@ static int build_maps_and_lists(pastix_data_t *pd) {
         L.upds0 = (int)pd->upd_tiles32.size();
         std::vector<pgpu::UpdTile> tc_far, s32_far;  // tiles whose target is two or more levels up
         L.upi0 = (int)pd->upd_i8_tiles.size();
+        std::vector<pgpu::UpdTile> i8_far;
         L.isl0 = (int)pd->i8_slabs.size();
         // FP64 tasks of the integer kernel: their DMMA / FMA tiles go to the end of the
         // lists, where a factorization whose images do not fit the device finds them
@@ -1322,15 +1323,18 @@ static int build_maps_and_lists(pastix_data_t *pd) {
                     if (!i8) continue;
                     const idx_t ra = tk.row0 + (side ? tk.n : 0);
                     const idx_t mi = (ra % 8 + M + 127) / 128, ni = (tk.row0 % 8 + tk.n + 127) / 128;
+                    const bool near = sv.cb_level[tk.dst] == (idx_t)l + 1;
                     for (idx_t a = 0; a < mi; a++)
                         for (idx_t c = 0; c < ni; c++)
                             if (fk == pgpu::FACT_GETRF || (a + 1) * 128 > c * 128)
-                                pd->upd_i8_tiles.push_back(pgpu::UpdTile{(int)t, (int)a, (int)c, side});
+                                (near ? pd->upd_i8_tiles : i8_far).push_back(pgpu::UpdTile{(int)t, (int)a, (int)c, side});
                 }
                 if (i8) pd->i8_off[tk.src] = 0;
             }
         }
-        {  // the images of a level's sources; the next level overwrites them
+        L.upin = (int)pd->upd_i8_tiles.size();
+        pd->upd_i8_tiles.insert(pd->upd_i8_tiles.end(), i8_far.begin(), i8_far.end());
+        {  // the images of a level's sources; the level after the next overwrites them
             int64_t bytes = 0;
             for (idx_t p = sv.lvl_ptr[l]; p < sv.lvl_ptr[l + 1]; p++) {
                 const idx_t k = sv.lvl_cblk[p];
@@ -1381,6 +1385,8 @@ static int build_maps_and_lists(pastix_data_t *pd) {
         L.updt1 = (int)pd->upd_tc_tiles.size();
         L.upds1 = (int)pd->upd_tiles32.size();
     }
+    for (idx_t k = 0; k < sv.cblknbr; k++)  // even and odd levels have an image area each
+        if (pd->i8_off[k] >= 0 && (sv.cb_level[k] & 1)) pd->i8_off[k] += pd->i8_total;
     return PASTIX_SUCCESS;
 }
 
@@ -1488,8 +1494,11 @@ static int device_setup(pastix_data_t *pd) {
     }
     if (d.dev < 0) CUDA_TRY(cudaGetDevice(&d.dev));
     CUDA_TRY(cudaSetDevice(d.dev));
-    if (!d.stream) CUDA_TRY(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
-    if (!d.side) CUDA_TRY(cudaStreamCreateWithFlags(&d.side, cudaStreamNonBlocking));
+    // the level chain's kernels go ahead of the far updates' remaining blocks
+    int plo = 0, phi = 0;
+    CUDA_TRY(cudaDeviceGetStreamPriorityRange(&plo, &phi));
+    if (!d.stream) CUDA_TRY(cudaStreamCreateWithPriority(&d.stream, cudaStreamNonBlocking, phi));
+    if (!d.side) CUDA_TRY(cudaStreamCreateWithPriority(&d.side, cudaStreamNonBlocking, plo));
     for (auto &e : d.ev_fact)
         if (!e) CUDA_TRY(cudaEventCreate(&e));
     while (d.ev_chain.size() < pd->levels.size()) {
@@ -1602,21 +1611,23 @@ struct PdlScope {
 // numerical factorization
 // ---------------------------------------------------------------------------
 template <typename T, int F>
-static int run_factor(pastix_data_t *pd) {
+static int run_factor(pastix_data_t *pd, bool overlap) {
     Device &d = pd->dev;
     cudaStream_t st = d.stream;
     T *L = reinterpret_cast<T *>(d.Lc.p);
     T *U = reinterpret_cast<T *>(d.Uc.p);
     T *Dinv = reinterpret_cast<T *>(d.dinv.p);
     pgpu::FactParams fp{d.crit.p, d.counters.p, d.counters.p + 1, d.dcscr.p};
-    // FP32: the updates of level l whose targets sit two or more levels up run on a
-    // second stream and overlap level l + 1 (all FP32 update writes are reductions)
-    // (the profiled pass keeps one stream so that each class's events time it alone)
-    const bool two = sizeof(T) == 4 && !pd->prof_on;
+    // the tensor-core updates of level l whose targets sit two or more levels up run
+    // on a second stream and overlap level l + 1 (every update write is a reduction
+    // then).  The profiled pass keeps one stream so that each class's events time it alone
+    const bool two = overlap && !pd->prof_on;
+    pgpu::DevStruct ds = d.ds;
+    ds.excl = !two;
     const cudaStream_t sd = two ? d.side : st;
     // FP32 (launched kernel by kernel, not as a graph): each launch of the level
     // chain overlaps the end of the kernel ahead of it (programmatic dependent launch)
-    PdlScope pdl_scope(two);
+    PdlScope pdl_scope(two && sizeof(T) == 4);
     if (sizeof(T) == 4 || d.i8_on)
         CUDA_TRY(cudaMemsetAsync(d.queues.p, 0, 3 * pd->levels.size() * sizeof(int), st));
     if (two) {
@@ -1627,58 +1638,58 @@ static int run_factor(pastix_data_t *pd) {
         const LevelLists &lv = pd->levels[l];
         if (two && l >= 2) CUDA_TRY(cudaStreamWaitEvent(st, d.ev_rest[l - 2], 0));
         launch_cls(pd, PC_PANEL_SMALL, lv.small1 - lv.small0, [&] {
-            pgpu::launch_panel_small<T, F>(d.ds, d.small_list.p + lv.small0, lv.small1 - lv.small0,
+            pgpu::launch_panel_small<T, F>(ds, d.small_list.p + lv.small0, lv.small1 - lv.small0,
                                            (size_t)pgpu::panel_small_bytes((long long)lv.small_smem_elems,
                                                                            (int)sizeof(T), lv.small_maxst),
                                            L, U, fp, st);
         });
         launch_cls(pd, PC_DIAG_LARGE, lv.large1 - lv.large0, [&] {
-            pgpu::launch_diag_large<T, F>(d.ds, d.large_list.p + lv.large0, lv.large1 - lv.large0, lv.diag_maxnc,
+            pgpu::launch_diag_large<T, F>(ds, d.large_list.p + lv.large0, lv.large1 - lv.large0, lv.diag_maxnc,
                                           lv.diag_smem_elems * sizeof(T), L, U, Dinv, fp, st);
         });
         if constexpr (sizeof(T) == 8) {
             launch_cls(pd, PC_TRSM, lv.trsm1 - lv.trsm0, [&] {
-                pgpu::launch_trsm<T, F>(d.ds, d.trsm_tiles.p + lv.trsm0, lv.trsm1 - lv.trsm0, lv.trsm_maxnc,
+                pgpu::launch_trsm<T, F>(ds, d.trsm_tiles.p + lv.trsm0, lv.trsm1 - lv.trsm0, lv.trsm_maxnc,
                                         lv.trsm_smem_elems * sizeof(T), L, U, Dinv, st);
             });
         } else {
             // FP32: X = A T^{-1} on tcgen05 -- inverses, their images, the panels' images before the TRSM
             launch_cls(pd, PC_TRSM, lv.tt1 - lv.tt0, [&] {
-                pgpu::launch_trinv<F>(d.ds, d.large_list.p + lv.large0, lv.large1 - lv.large0, lv.ti_maxnzb, L, U,
+                pgpu::launch_trinv<F>(ds, d.large_list.p + lv.large0, lv.large1 - lv.large0, lv.ti_maxnzb, L, U,
                                       Dinv, d.ti_off.p, d.tinv.p, st);
                 pgpu::launch_split_dense(d.dense_slabs.p + lv.ds0, lv.ds1 - lv.ds0, d.tinv.p, d.timg.p, st);
                 const pgpu::SplitSlab *sl = d.split_slabs.p + lv.spl0;
                 const int cnt = lv.spl1 - lv.spl0;
-                pgpu::launch_split(d.ds, sl, cnt, L, L, d.sp_off.p, d.img0.p, 0, st);
-                if (F == pgpu::FACT_GETRF) pgpu::launch_split(d.ds, sl, cnt, U, L, d.sp_off.p, d.img1.p, 0, st);
-                pgpu::launch_trsm_tc<F>(d.ds, d.trsm_tc_tiles.p + lv.tt0, lv.tt1 - lv.tt0, L, U, d.img0.p, d.img1.p,
+                pgpu::launch_split(ds, sl, cnt, L, L, d.sp_off.p, d.img0.p, 0, st);
+                if (F == pgpu::FACT_GETRF) pgpu::launch_split(ds, sl, cnt, U, L, d.sp_off.p, d.img1.p, 0, st);
+                pgpu::launch_trsm_tc<F>(ds, d.trsm_tc_tiles.p + lv.tt0, lv.tt1 - lv.tt0, L, U, d.img0.p, d.img1.p,
                                         d.sp_off.p, d.timg.p, d.ti_img.p, d.queues.p + 3 * l, d.counters.p + 1, st);
             });
             launch_cls(pd, PC_TRSM, lv.tr32_1 - lv.tr32_0, [&] {
-                pgpu::launch_trsm<T, F>(d.ds, d.trsm_tiles32.p + lv.tr32_0, lv.tr32_1 - lv.tr32_0, lv.trsm_maxnc,
+                pgpu::launch_trsm<T, F>(ds, d.trsm_tiles32.p + lv.tr32_0, lv.tr32_1 - lv.tr32_0, lv.trsm_maxnc,
                                         lv.trsm_smem_elems * sizeof(T), L, U, Dinv, st);
             });
         }
         if constexpr (sizeof(T) == 8) {
             const int n = (d.i8_on ? lv.updm : lv.upd1) - lv.upd0;
             launch_cls(pd, PC_UPDATE, n, [&] {
-                pgpu::launch_update<T, F>(d.ds, d.upd_tiles.p + lv.upd0, n, L, U, st);
+                pgpu::launch_update<T, F>(ds, d.upd_tiles.p + lv.upd0, n, L, U, st);
             });
         } else {
             launch_cls(pd, PC_UPDATE, lv.updsn - lv.upds0, [&] {
-                pgpu::launch_update<T, F>(d.ds, d.upd_tiles32.p + lv.upds0, lv.updsn - lv.upds0, L, U, st);
+                pgpu::launch_update<T, F>(ds, d.upd_tiles32.p + lv.upds0, lv.updsn - lv.upds0, L, U, st);
             });
         }
         if constexpr (sizeof(T) == 4) {
             launch_cls(pd, PC_SPLIT, lv.spl1 - lv.spl0, [&] {
                 const pgpu::SplitSlab *sl = d.split_slabs.p + lv.spl0;
                 const int cnt = lv.spl1 - lv.spl0;
-                pgpu::launch_split(d.ds, sl, cnt, L, L, d.sp_off.p, d.img0.p, 0, st);
-                if (F == pgpu::FACT_SYTRF) pgpu::launch_split(d.ds, sl, cnt, L, L, d.sp_off.p, d.img1.p, 1, st);
-                if (F == pgpu::FACT_GETRF) pgpu::launch_split(d.ds, sl, cnt, U, L, d.sp_off.p, d.img1.p, 0, st);
+                pgpu::launch_split(ds, sl, cnt, L, L, d.sp_off.p, d.img0.p, 0, st);
+                if (F == pgpu::FACT_SYTRF) pgpu::launch_split(ds, sl, cnt, L, L, d.sp_off.p, d.img1.p, 1, st);
+                if (F == pgpu::FACT_GETRF) pgpu::launch_split(ds, sl, cnt, U, L, d.sp_off.p, d.img1.p, 0, st);
             });
             launch_cls(pd, PC_UPDATE_BIG, lv.updtn - lv.updt0, [&] {
-                pgpu::launch_update_tc<F>(d.ds, d.upd_tc_tiles.p + lv.updt0, lv.updtn - lv.updt0, L, U, d.img0.p,
+                pgpu::launch_update_tc<F>(ds, d.upd_tc_tiles.p + lv.updt0, lv.updtn - lv.updt0, L, U, d.img0.p,
                                           d.img1.p, d.sp_off.p, d.queues.p + 3 * l + 1, d.counters.p + 1, st);
             });
             // far targets on the side stream, once this level's panels and images are final
@@ -1689,13 +1700,13 @@ static int run_factor(pastix_data_t *pd) {
             launch_cls(
                 pd, PC_UPDATE, lv.upds1 - lv.updsn,
                 [&] {
-                    pgpu::launch_update<T, F>(d.ds, d.upd_tiles32.p + lv.updsn, lv.upds1 - lv.updsn, L, U, sd);
+                    pgpu::launch_update<T, F>(ds, d.upd_tiles32.p + lv.updsn, lv.upds1 - lv.updsn, L, U, sd);
                 },
                 sd);
             launch_cls(
                 pd, PC_UPDATE_BIG, lv.updt1 - lv.updtn,
                 [&] {
-                    pgpu::launch_update_tc<F>(d.ds, d.upd_tc_tiles.p + lv.updtn, lv.updt1 - lv.updtn, L, U,
+                    pgpu::launch_update_tc<F>(ds, d.upd_tc_tiles.p + lv.updtn, lv.updt1 - lv.updtn, L, U,
                                               d.img0.p, d.img1.p, d.sp_off.p, d.queues.p + 3 * l + 2,
                                               d.counters.p + 1, sd);
                 },
@@ -1704,24 +1715,38 @@ static int run_factor(pastix_data_t *pd) {
         } else {
             const int n = (d.i8_on ? lv.updbm : lv.updb1) - lv.updb0;
             launch_cls(pd, PC_UPDATE_BIG, n, [&] {
-                pgpu::launch_update_big<T, F>(d.ds, d.upd_big_tiles.p + lv.updb0, n, L, U, st);
+                pgpu::launch_update_big<T, F>(ds, d.upd_big_tiles.p + lv.updb0, n, L, U, st);
             });
             if (d.i8_on) {
                 const int nsl = lv.isl1 - lv.isl0;
                 launch_cls(pd, PC_SPLIT, nsl, [&] {
                     const pgpu::SplitSlab *sl = d.i8_slabs.p + lv.isl0;
-                    pgpu::launch_split_i8(d.ds, sl, nsl, L, L, d.i8_off.p, d.i8_img0.p, d.i8_sc0.p,
+                    pgpu::launch_split_i8(ds, sl, nsl, L, L, d.i8_off.p, d.i8_img0.p, d.i8_sc0.p,
                                           F == pgpu::FACT_POTRF ? 0 : 1, st);
                     if (F == pgpu::FACT_SYTRF)
-                        pgpu::launch_split_i8(d.ds, sl, nsl, L, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 2, st);
+                        pgpu::launch_split_i8(ds, sl, nsl, L, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 2, st);
                     if (F == pgpu::FACT_GETRF)
-                        pgpu::launch_split_i8(d.ds, sl, nsl, U, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 3, st);
+                        pgpu::launch_split_i8(ds, sl, nsl, U, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 3, st);
                 });
-                launch_cls(pd, PC_UPDATE_BIG, lv.upi1 - lv.upi0, [&] {
-                    pgpu::launch_update_i8<F>(d.ds, d.upd_i8_tiles.p + lv.upi0, lv.upi1 - lv.upi0, L, U, d.i8_img0.p,
+                const int nnear = (two ? lv.upin : lv.upi1) - lv.upi0;
+                launch_cls(pd, PC_UPDATE_BIG, nnear, [&] {
+                    pgpu::launch_update_i8<F>(ds, d.upd_i8_tiles.p + lv.upi0, nnear, L, U, d.i8_img0.p,
                                               d.i8_img1.p, d.i8_sc0.p, d.i8_sc1.p, d.i8_off.p, d.queues.p + 3 * l,
-                                              d.counters.p + 1, pgpu::sm_count(), st);
+                                              d.counters.p + 1, false, st);
                 });
+                if (two) {
+                    CUDA_TRY(cudaEventRecord(d.ev_chain[l], st));
+                    CUDA_TRY(cudaStreamWaitEvent(d.side, d.ev_chain[l], 0));
+                    launch_cls(
+                        pd, PC_UPDATE_BIG, lv.upi1 - lv.upin,
+                        [&] {
+                            pgpu::launch_update_i8<F>(ds, d.upd_i8_tiles.p + lv.upin, lv.upi1 - lv.upin, L, U,
+                                                      d.i8_img0.p, d.i8_img1.p, d.i8_sc0.p, d.i8_sc1.p, d.i8_off.p,
+                                                      d.queues.p + 3 * l + 2, d.counters.p + 1, true, sd);
+                        },
+                        sd);
+                    CUDA_TRY(cudaEventRecord(d.ev_rest[l], d.side));
+                }
             }
         }
     }
@@ -1862,7 +1887,7 @@ extern "C" int pastix_subtask_bcsc2ctab(pastix_data_t *pd) {
     // FP64: digit images of one level's panels; a factorization for which they do not fit runs on DMMA
     d.i8_on = false;
     if (!pd->mixed && pd->i8_total > 0) {
-        const size_t ib = (size_t)pd->i8_total, nr = pd->solver.rowidx.size();
+        const size_t ib = 2 * (size_t)pd->i8_total, nr = pd->solver.rowidx.size();
         const bool two = fk != pgpu::FACT_POTRF;
         d.i8_on = d.i8_img0.alloc(ib) == cudaSuccess && d.i8_sc0.alloc(nr) == cudaSuccess &&
                   (!two || (d.i8_img1.alloc(ib) == cudaSuccess && d.i8_sc1.alloc(nr) == cudaSuccess));
@@ -1911,19 +1936,28 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
         // FP32 factors: launched kernel by kernel.  Replayed as a graph, the same launches ran
         // 12% slower on a B200 (100^3 Laplacian: 83 ms against 74 ms, with or without the side
         // stream in the graph), so only the solves of this precision are graphed.
-        if (fk == pgpu::FACT_POTRF) rc = run_factor<float, pgpu::FACT_POTRF>(pd);
-        else if (fk == pgpu::FACT_SYTRF) rc = run_factor<float, pgpu::FACT_SYTRF>(pd);
-        else rc = run_factor<float, pgpu::FACT_GETRF>(pd);
+        if (fk == pgpu::FACT_POTRF) rc = run_factor<float, pgpu::FACT_POTRF>(pd, true);
+        else if (fk == pgpu::FACT_SYTRF) rc = run_factor<float, pgpu::FACT_SYTRF>(pd, true);
+        else rc = run_factor<float, pgpu::FACT_GETRF>(pd, true);
     } else {
-        // FP64: the whole level sequence is one CUDA graph per (kind, buffers)
-        const std::vector<uintptr_t> key{1, (uintptr_t)fk, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p,
-                                         (uintptr_t)d.i8_img0.p, (uintptr_t)d.i8_img1.p, (uintptr_t)d.i8_sc0.p,
-                                         (uintptr_t)d.i8_sc1.p};
-        rc = run_graphed(pd, key, [&]() -> int {
-            if (fk == pgpu::FACT_POTRF) return run_factor<double, pgpu::FACT_POTRF>(pd);
-            if (fk == pgpu::FACT_SYTRF) return run_factor<double, pgpu::FACT_SYTRF>(pd);
-            return run_factor<double, pgpu::FACT_GETRF>(pd);
-        });
+        // FP64: large factorizations overlap a level's far updates with the next level's
+        // panels and are launched kernel by kernel (in a graph the streams' priorities are
+        // lost: 60^3 Laplacian 16.2 ms, 13.9 launched, 15.7 as a graph on one stream); small
+        // ones are one CUDA graph per (kind, buffers) (20^3: 0.62 ms against 0.68 launched)
+        const bool overlap = d.i8_on && pd->solver.thflops >= 2e10;
+        auto run = [&]() -> int {
+            if (fk == pgpu::FACT_POTRF) return run_factor<double, pgpu::FACT_POTRF>(pd, overlap);
+            if (fk == pgpu::FACT_SYTRF) return run_factor<double, pgpu::FACT_SYTRF>(pd, overlap);
+            return run_factor<double, pgpu::FACT_GETRF>(pd, overlap);
+        };
+        if (overlap) {
+            rc = run();
+        } else {
+            const std::vector<uintptr_t> key{1, (uintptr_t)fk, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p,
+                                             (uintptr_t)d.i8_img0.p, (uintptr_t)d.i8_img1.p, (uintptr_t)d.i8_sc0.p,
+                                             (uintptr_t)d.i8_sc1.p};
+            rc = run_graphed(pd, key, run);
+        }
     }
     if (rc) return rc;
     int cnt[2] = {0, 0};

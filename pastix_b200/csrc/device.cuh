@@ -72,6 +72,7 @@ struct DevStruct {
     const int *bk_frow, *bk_lrow, *bk_rowoff, *bk_fcblk;
     const int *rowidx;          // global row of every panel row
     const TaskDev *tasks;
+    int excl;                   // exclusive targets may be written without reductions (no updates of two levels at once)
 };
 
 // Per-call scalars for the factorization kernels.

@@ -26,6 +26,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 
 namespace pgpu {
 
@@ -809,7 +810,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
             int rr = rt[tx + i * TX];
             dst[i] = (rr < 0) ? nullptr : Cp + rr + (size_t)cc * stf;
         }
-        if (tk.excl && sizeof(T) == 8) {  // FP32 updates of different levels may overlap: reductions only
+        if (tk.excl && s.excl) {
             T old[TM];
 #pragma unroll
             for (int i = 0; i < TM; i++) old[i] = dst[i] ? *dst[i] : T(0);
@@ -955,7 +956,7 @@ __global__ void __launch_bounds__(256) k_update_dmma(DevStruct s, const UpdTile 
                 const int cc = ct[wn + j * 8 + q4 * 2 + h];
                 dst[j * 2 + h] = (cc < 0) ? nullptr : Cp + rr + (size_t)cc * stf;
             }
-        if (tk.excl) {
+        if (tk.excl && s.excl) {
             double old[8];
 #pragma unroll
             for (int q = 0; q < 8; q++) old[q] = dst[q] ? *dst[q] : 0.0;
@@ -3033,6 +3034,14 @@ void launch_update_big(const DevStruct &s, const UpdTile *tiles, int count, T *L
         k_update<T, FACT, 128, 64, 16, 8, 4><<<count, 256, 0, st>>>(s, tiles, L, U);
 }
 
+// CTAs of a persistent update kernel, each of at most `quota` tiles (INT_MAX: one
+// per SM until the tiles are done).  The FP64 updates of far targets run beside the
+// next level's panels on a stream of lower priority; a persistent launch there
+// would keep those panels waiting for its end.
+int far_grid(int count, int quota) {
+    const int full = std::min(count, sm_count());
+    return quota == INT_MAX ? full : std::max(full, (count + quota - 1) / quota);
+}
 // FP32 updates of 128 x 128 tiles on tcgen05 from the split BF16 images
 template <int FACT>
 void launch_update_tc(const DevStruct &s, const UpdTile *tiles, int count, float *L, float *U,

@@ -31,7 +31,7 @@
 #include "device.cuh"
 #include "tcgen05.cuh"
 
-#include <algorithm>
+#include <climits>
 
 namespace pgpu {
 
@@ -46,10 +46,14 @@ constexpr int I8_THREADS = 320;            // 8 epilogue warps, producer, MMA is
 constexpr int I8_EPI = 256;
 constexpr int I8_BN = 128;
 constexpr int I8_TQ = 4;                   // tile-index ring
+constexpr int FAR_TILES_I8 = 6;            // tiles of a CTA of the far updates, about 80 us: 60^3 Laplacian,
+                                           // factorization 15.7 -> 13.9 ms against one stream (far_grid)
 constexpr int I8_MAX_K = 512;              // widest source: the low part of the sums stays within 2^50
 
 __host__ __device__ inline int i8_nkb(int nc) { return (nc + I8_KB - 1) / I8_KB; }
 __host__ __device__ inline int i8_ng(int st) { return (st + 7) / 8 + 16; }
+
+int far_grid(int count, int quota);  // factor.cu
 
 long long i8_image_bytes(int nc, int st) { return (long long)I8_S * i8_nkb(nc) * i8_ng(st) * I8_GROUP; }
 int i8_max_k() { return I8_MAX_K; }
@@ -224,7 +228,7 @@ __device__ __forceinline__ int i8_bar_or(int pred) {  // OR over the epilogue th
 
 template <int FACT>
 __global__ void __launch_bounds__(I8_THREADS, 1)
-    k_update_i8(DevStruct s, const UpdTile *__restrict__ tiles, int count, double *L, double *U,
+    k_update_i8(DevStruct s, const UpdTile *__restrict__ tiles, int count, int quota, double *L, double *U,
                 const unsigned char *img0, const unsigned char *img1, const double *__restrict__ sc0,
                 const double *__restrict__ sc1, const int64_t *__restrict__ i8_off, int *queue, int *status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -269,8 +273,8 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
                     break;
                 }
                 int t = next;
-                if (t >= count) t = -1;
-                else next = atomicAdd(queue, 1);
+                if (t >= count || j >= quota) t = -1;  // `quota`: tiles of this CTA
+                else if (j + 1 < quota) next = atomicAdd(queue, 1);
                 tq[slot] = t;
                 mbar_arrive(&tq_full[slot]);
                 if (t < 0) break;
@@ -463,10 +467,11 @@ void launch_split_i8(const DevStruct &s, const SplitSlab *slabs, int count, cons
 template <int FACT>
 void launch_update_i8(const DevStruct &s, const UpdTile *tiles, int count, double *L, double *U,
                       const unsigned char *img0, const unsigned char *img1, const double *sc0, const double *sc1,
-                      const int64_t *i8_off, int *queue, int *status, int sms, cudaStream_t st) {
+                      const int64_t *i8_off, int *queue, int *status, bool far, cudaStream_t st) {
     if (count <= 0) return;
-    k_update_i8<FACT><<<std::min(count, sms), I8_THREADS, I8_SMEM, st>>>(s, tiles, count, L, U, img0, img1, sc0, sc1,
-                                                                         i8_off, queue, status);
+    const int quota = far ? FAR_TILES_I8 : INT_MAX;
+    k_update_i8<FACT><<<far_grid(count, quota), I8_THREADS, I8_SMEM, st>>>(s, tiles, count, quota, L, U, img0, img1, sc0,
+                                                                           sc1, i8_off, queue, status);
 }
 cudaError_t set_i8_attrs() {
     cudaError_t e = cudaSuccess;
@@ -477,7 +482,7 @@ cudaError_t set_i8_attrs() {
 #define PGPU_INST_I8(F)                                                                                               \
     template void launch_update_i8<F>(const DevStruct &, const UpdTile *, int, double *, double *,                    \
                                       const unsigned char *, const unsigned char *, const double *, const double *,   \
-                                      const int64_t *, int *, int *, int, cudaStream_t);
+                                      const int64_t *, int *, int *, bool, cudaStream_t);
 PGPU_INST_I8(FACT_POTRF)
 PGPU_INST_I8(FACT_SYTRF)
 PGPU_INST_I8(FACT_GETRF)
