@@ -4,15 +4,23 @@
 // The product C -= A B^T of an update task is formed from fixed-point operands
 // (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms
 // 59, 2012, with a common exponent per row): k_split_i8 scales every panel row
-// by a power of two, rounds it to 55 fractional bits below the row's largest
-// entry and cuts the integer into seven signed 8-bit digits (balanced base
+// by a power of two, rounds it to 63 fractional bits below the row's largest
+// entry and cuts the integer into eight signed 8-bit digits (balanced base
 // 256).  Products of digits and their sums over up to I8_MAX_K columns are
-// exact in 32 bits; the digit products i, j with i + j <= 7 are kept (34 of
-// 49).  What is dropped -- 2^-64 of the largest products of a row pair, and the
-// rounding of entries smaller than 1/4 of their row's largest -- lies below the
-// rounding of the K additions that an FP64 accumulation of the same product
-// makes; the sums of the kept products are exact and are rounded once.  Rows
-// with a non-finite entry carry a NaN scale, so that it reaches the target.
+// exact in 32 bits; the digit products i, j with i + j <= 7 are kept (36 of
+// 64).  What is lost, with a and b the scales of the two rows (the powers of two
+// above their largest entries):
+//   entries smaller than 2^-10 a are rounded at 2^-64 a, the others are exact;
+//   the dropped digit products come to about 2^-60 a b for 128 columns of equal
+//   size (at most 2^-61 a b for each column); the sums i + j >= 4 are rounded at
+//   2^-60 a b, and the whole sum once to FP64.
+// So the error is bounded against a b, not against the sum of the |a_c b_c| that
+// bounds FP64 accumulation: for Cholesky a b <= 4 sqrt(A_ii A_jj), the bound that
+// its FP64 rounding has, with 2^-60 in place of K 2^-53.  Rows with a non-finite
+// entry carry a NaN scale, so that it reaches the target.
+// Measured against the factor in 64-bit mantissas (full 520 x 520 kernel matrix
+// with shuffled rows, panels of 64): FP64 on DMMA 3.3e-14, here 1.8e-14; seven
+// digits with the low sums rounded at 2^-51 a b gave 2.4e-13.
 // Rounding relative to the row's largest entry asks for columns of like size:
 // the rows of a Cholesky factor are bounded by the diagonal of A, those of L in
 // LDL^T and LU are not (a small pivot makes a large column).  There column c is
@@ -20,7 +28,7 @@
 // and (L h)(U / h), the balance that Cholesky has.
 //
 // Why: the FP64 tensor cores (DMMA) multiply 64 x 2 flops per clock and SM, the
-// 8-bit ones 8192 x 2; 34 digit products per FP64 product are 3.8 times fewer
+// 8-bit ones 8192 x 2; 36 digit products per FP64 product are 3.6 times fewer
 // tensor-core cycles.  Rates measured are given at k_update_i8.
 //
 // Image of cblk k (bytes from i8_off[k]): digit p (0 the leading one), K block
@@ -35,7 +43,8 @@
 
 namespace pgpu {
 
-constexpr int I8_S = 7;                    // digits
+constexpr int I8_S = 8;                    // digits
+constexpr int I8_BITS = 8 * I8_S - 1;      // fractional bits below a row's largest entry
 constexpr int I8_KB = 32;                  // columns per K block (one MMA step)
 constexpr int I8_GROUP = 256;              // bytes of 8 rows x 32 columns of one digit
 constexpr int I8_PIECE = 16 * I8_GROUP;    // one digit of a 128-row operand block
@@ -48,7 +57,7 @@ constexpr int I8_BN = 128;
 constexpr int I8_TQ = 4;                   // tile-index ring
 constexpr int FAR_TILES_I8 = 6;            // tiles of a CTA of the far updates, about 80 us: 60^3 Laplacian,
                                            // factorization 15.7 -> 13.9 ms against one stream (far_grid)
-constexpr int I8_MAX_K = 512;              // widest source: the low part of the sums stays within 2^50
+constexpr int I8_MAX_K = 512;              // widest source: the sums i + j >= 4 stay within 2^50
 
 __host__ __device__ inline int i8_nkb(int nc) { return (nc + I8_KB - 1) / I8_KB; }
 __host__ __device__ inline int i8_ng(int st) { return (st + 7) / 8 + 16; }
@@ -64,7 +73,7 @@ int i8_max_k() { return I8_MAX_K; }
 // largest magnitude, the second (the slab is in L1 / L2 by then) writes the
 // digits, 16 bytes per digit and chunk.  Column factors by `mode`: 0 none, 1 h_c,
 // 2 D_c / h_c, 3 1 / h_c, with D_c the pivot on the diagonal of panel Dp.  Bound
-// by HBM: 8 bytes read and 7 written per entry.
+// by HBM: 8 bytes read and 8 written per entry.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *__restrict__ slabs, const double *P,
                                                   const double *Dp, const int64_t *__restrict__ i8_off,
@@ -128,10 +137,11 @@ __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *
     }
     // row exponent: |a| < 127.375 / 128 * 2^ex, so that the leading digit fits 8
     // bits after the carries of the balanced digits (at most 0.502 of it)
-    int ex = ((__double2hiint(m) >> 20) & 0x7ff) - 1022;
-    if (ex < -900) ex = -900;  // rows below 2^-900: absolute rounding
-    if (!bad && m >= 0.9951171875 * pow2(ex - 1) * 2.0) ex++;
-    const double mult = bad ? 0.0 : pow2(55 - ex);
+    const int mhi = __double2hiint(m);
+    int ex = ((mhi >> 20) & 0x7ff) - 1022;
+    if ((mhi & 0xfffff) >= 0xfd800) ex++;  // mantissa of 2 * 127.375 / 128
+    if (ex < -958) ex = -958;              // smaller rows: rounded at 2^-1021, as subnormal numbers are
+    const double mult = bad ? 0.0 : pow2(I8_BITS - ex);
     if (warp == 0 && pr < st)
         rscale[s.cb_rowidx[k] + pr] = bad ? __longlong_as_double(0x7ff8000000000000LL) : pow2(ex - 19);
     if (pr >= 8 * ((st + 7) / 8)) return;
@@ -146,7 +156,7 @@ __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const long long q = bad ? 0 : __double2ll_rn(v[4 * g + j] * mult);
-                const unsigned long long t = (unsigned long long)(q + 0x808080808080LL);
+                const unsigned long long t = (unsigned long long)q + 0x80808080808080ULL;
                 lo[j] = (uint32_t)t;
                 hi[j] = (uint32_t)(t >> 32);
             }
@@ -155,13 +165,14 @@ __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *
             const uint32_t l01b = __byte_perm(lo[0], lo[1], 0x7362), l23b = __byte_perm(lo[2], lo[3], 0x7362);
             const uint32_t h01a = __byte_perm(hi[0], hi[1], 0x5140), h23a = __byte_perm(hi[2], hi[3], 0x5140);
             const uint32_t h01b = __byte_perm(hi[0], hi[1], 0x7362), h23b = __byte_perm(hi[2], hi[3], 0x7362);
-            w[6][g] = __byte_perm(l01a, l23a, 0x5410) ^ 0x80808080u;
-            w[5][g] = __byte_perm(l01a, l23a, 0x7632) ^ 0x80808080u;
-            w[4][g] = __byte_perm(l01b, l23b, 0x5410) ^ 0x80808080u;
-            w[3][g] = __byte_perm(l01b, l23b, 0x7632) ^ 0x80808080u;
-            w[2][g] = __byte_perm(h01a, h23a, 0x5410) ^ 0x80808080u;
-            w[1][g] = __byte_perm(h01a, h23a, 0x7632) ^ 0x80808080u;
-            w[0][g] = __byte_perm(h01b, h23b, 0x5410);
+            w[7][g] = __byte_perm(l01a, l23a, 0x5410) ^ 0x80808080u;
+            w[6][g] = __byte_perm(l01a, l23a, 0x7632) ^ 0x80808080u;
+            w[5][g] = __byte_perm(l01b, l23b, 0x5410) ^ 0x80808080u;
+            w[4][g] = __byte_perm(l01b, l23b, 0x7632) ^ 0x80808080u;
+            w[3][g] = __byte_perm(h01a, h23a, 0x5410) ^ 0x80808080u;
+            w[2][g] = __byte_perm(h01a, h23a, 0x7632) ^ 0x80808080u;
+            w[1][g] = __byte_perm(h01b, h23b, 0x5410) ^ 0x80808080u;
+            w[0][g] = __byte_perm(h01b, h23b, 0x7632);
         }
         unsigned char *o = out + (size_t)(ch >> 1) * ng * I8_GROUP + (ch & 1) * 128;
 #pragma unroll
@@ -174,16 +185,17 @@ __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *
 // The tile kernel: persistent, warp specialized, tiles from a device work queue
 // as in the FP32 engine.  128 x 128 tiles; the eight digit sums d = i + j do not
 // fit the 512 tensor-memory columns at once, so that a tile takes two passes
-// over K: first d = 4..7 (24 digit products, seven digits of each operand), kept
-// by the epilogue threads as 31-bit integers, then d = 0..3 (10 products, four
+// over K: first d = 4..7 (26 digit products, eight digits of each operand), kept
+// by the epilogue threads as 40-bit integers, then d = 0..3 (10 products, four
 // digits), added and scattered into the facing panel.  N = 128 rather than 64
 // with all sums resident: at N = 64 the tensor cores read shared memory faster
 // than it delivers (192 bytes a clock).
 // 100^3 Laplacian, B200, all updates of an FP64 factorization: 264 ms on DMMA
-// (k_update_dmma, 23 Tflop/s), 111 ms here (55 Tflop/s).  Bounds, 80^3: copies
+// (k_update_dmma, 23 Tflop/s), 118 ms here (52 Tflop/s; 112 with seven digits).
+// 80^3: 33.8 ms.  Bounds there, with seven digits (whole kernel 31.8): copies
 // alone 22.9 ms (L2 to shared memory, 35 bytes a clock and SM), products and
-// hand-offs alone 22.2 (tensor pipe 14.7), both without epilogue 24.0, with it
-// 31.8.  Slower: 16 or 8 epilogue warps that release the accumulators before
+// hand-offs alone 22.2 (tensor pipe 14.3), both without epilogue 24.0.
+// Slower: 16 or 8 epilogue warps that release the accumulators before
 // they scatter (33.1, 37.2: the registers spill), one polling lane per warp (34.7).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t i8_desc(uint32_t saddr) {
@@ -346,9 +358,9 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
 #pragma unroll
                             for (int d = 4; d < 8; d++)
 #pragma unroll
-                                for (int p = d - 6 > 0 ? d - 6 : 0; p <= (d < 6 ? d : 6); p++)
+                                for (int p = 0; p <= d; p++)
                                     i8_mma(tmem + I8_BN * (d - 4), da + p * (I8_PIECE >> 4), db + (d - p) * (I8_PIECE >> 4),
-                                           idesc, kb > 0 || p > (d - 6 > 0 ? d - 6 : 0));
+                                           idesc, kb > 0 || p > 0);
                         } else {
 #pragma unroll
                             for (int d = 0; d < 4; d++)
@@ -411,14 +423,21 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
             }
             tc_fence_after();
             ph++;
-            int low[64];  // the sums d = 4..7 in units of 2^20 of the last digit's
+            // the sums d = 4..7 in units of 2^11 of the last digit's, 40 bits: upper 32 and lower 8
+            int low[64];
+            uint32_t lob[16];
 #pragma unroll
             for (int q = 0; q < 8; q++) {
                 if (cbase + 8 * q < nmma) {
                     long long z[8];
                     i8_load4(taddr + 8 * q, z);
 #pragma unroll
-                    for (int j = 0; j < 8; j++) low[8 * q + j] = (int)((z[j] + (1 << 19)) >> 20);
+                    for (int j = 0; j < 8; j++) {
+                        const long long r = (z[j] + (1 << 10)) >> 11;
+                        low[8 * q + j] = (int)(r >> 8);
+                        uint32_t &w = lob[2 * q + (j >> 2)];
+                        w = (j & 3) ? w | ((uint32_t)r & 255u) << 8 * (j & 3) : (uint32_t)r & 255u;
+                    }
                 }
             }
             tc_fence_before();
@@ -440,9 +459,10 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
                     for (int j = 0; j < 8; j++) {
                         // both integers to FP64 exactly (|z| < 2^51) by the offset of their magic exponents
                         const double h = __longlong_as_double(z[j] + 0x4338000000000000LL) - 6755399441055744.0;
-                        const double l = __hiloint2double(0x43300000, low[8 * q + j] ^ 0x80000000) - 4503601774854144.0;
+                        const long long r = (long long)low[8 * q + j] * 256 + ((lob[2 * q + (j >> 2)] >> 8 * (j & 3)) & 255u);
+                        const double l = __longlong_as_double(r + 0x4338000000000000LL) - 6755399441055744.0;
                         const int cc = ctab[b][cbase + 8 * q + j];
-                        const double v = fma(l, 0x1p-12, h) * rs * csc[b][cbase + 8 * q + j];
+                        const double v = fma(l, 0x1p-21, h) * (rs * csc[b][cbase + 8 * q + j]);
                         if (rr >= 0 && cc >= 0) atomicAdd(Cp + (size_t)cc * stf, v);
                     }
                 }

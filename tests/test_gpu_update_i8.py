@@ -12,9 +12,10 @@ import numpy as np
 import pytest
 import scipy.sparse as sps
 
-from conftest import analyse, backward_error
+from conftest import FACT_ID, analyse, backward_error
 from pastix_b200 import gen
 from pastix_b200 import pastix as px
+from pastix_b200.spm import mtxtype, spmatrix
 from test_gpu_parity import _mask_compare
 
 pytestmark = pytest.mark.gpu
@@ -63,6 +64,83 @@ def test_scaled_rows(lib, fact, decades):
     px.task_solve(pd, S, x)
     # in the unscaled unknowns the backward error is that of a stable solve of A
     assert backward_error(A, d * x, b / d) < 4e-13
+    px.finalize(pd)
+
+
+def _dense_chain(A, fact, width):
+    """Handle of a full matrix cut into panels of `width` columns, in the given order."""
+    n = A.shape[0]
+    ip, dp = px.initParam()
+    ip[px.iparm.factorization] = FACT_ID[fact]
+    pd = px.init(ip, dp)
+    S = spmatrix(sps.csc_matrix(A), mtxtype.General if fact == "GETRF" else mtxtype.Symmetric)
+    rang = np.append(np.arange(0, n, width), n).astype(np.int64)
+    tree = np.append(np.arange(1, len(rang) - 1), -1).astype(np.int64)
+    px.subtask_order(pd, S, np.arange(n), rang, tree)
+    px.subtask_symbfact(pd)
+    px.subtask_blend(pd)
+    return pd, S, px.solver_info(pd)
+
+
+def _dense_factor(info, panels):
+    """The lower triangle (with the diagonal) held in the panels of a full matrix."""
+    n = int(info["cb_lcol"][-1]) + 1
+    F = np.zeros((n, n))
+    for k in range(int(info["cblknbr"])):
+        fc, lc, st, base = (int(info[q][k]) for q in ("cb_fcol", "cb_lcol", "cb_stride", "cb_coef"))
+        for c in range(fc, lc + 1):
+            F[c:, c] = panels[base + (c - fc) * st + (c - fc): base + (c - fc + 1) * st]
+    return F
+
+
+def _lu(A, width):
+    """LU without pivoting in the precision of A, updates in panels of `width` columns (0: column by column)."""
+    A, n = A.copy(), len(A)
+    w = width or n
+    for k in range(0, n, w):
+        e = min(n, k + w)
+        for c in range(k, e):
+            A[c + 1:, c] /= A[c, c]
+            A[c + 1:, c + 1:e] -= np.outer(A[c + 1:, c], A[c, c + 1:e])
+        for c in range(k, e):
+            A[c, e:] -= A[c, k:c] @ A[k:c, e:]
+        A[e:, e:] -= A[e:, k:e] @ A[k:e, e:]
+    return A
+
+
+@pytest.mark.parametrize("fact", ["POTRF", "SYTRF", "GETRF"])
+@pytest.mark.parametrize("width", [64, 100])
+def test_updates_lose_nothing_against_fp64(lib, fact, width):
+    """A full matrix whose factor rows hold entries of many sizes that seldom face each other, against its
+    elimination in 64-bit mantissas.  Yardstick: the error of the same elimination in FP64; half as much
+    again is left for another order of its sums."""
+    rng = np.random.default_rng(0)
+    n = 520
+    q = rng.permutation(n)
+    A = np.exp(-np.abs(np.subtract.outer(q, q)) / 20.0) + 0.05 * np.eye(n)
+    if fact == "GETRF":
+        A *= 1.0 + 0.01 * np.random.default_rng(1).uniform(-1, 1, (n, n))
+    ref = _lu(A.astype(np.longdouble), 0)
+    e64 = (_lu(A, width) - ref).astype(float)
+    pd, S, info = _dense_chain(A, fact, width)
+    assert int((info["cb_lcol"] - info["cb_fcol"]).max()) + 1 == width
+    px.task_numfact(pd, S)
+    Lg, Ug = px.get_coeftab(pd, with_u=(fact == "GETRF"))
+    F = _dense_factor(info, Lg)
+    d = np.sqrt(np.diag(ref).astype(float))
+    if fact == "POTRF":
+        got, want = np.tril(F), np.tril(ref, -1) * d[None, :] + np.diag(d)
+        e64 = np.tril(e64, -1) * d[None, :]
+    else:
+        got, want = np.tril(F, -1), np.tril(ref, -1)
+        e64 = np.tril(e64, -1)
+    err = np.linalg.norm(np.tril((got - want).astype(float), -1))
+    assert err < 1.5 * np.linalg.norm(e64)
+    if fact == "GETRF":
+        Ut = np.tril(_dense_factor(info, Ug), -1)
+        e64 = np.triu((_lu(A, width) - ref).astype(float), 1)
+        err = np.linalg.norm(Ut - np.triu(ref, 1).T.astype(float))
+        assert err < 1.5 * np.linalg.norm(e64)
     px.finalize(pd)
 
 
