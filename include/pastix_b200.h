@@ -379,11 +379,22 @@ int pgpu_graphs(pastix_data_t *pastix_data, int enable);
  * simple refinement keep the column loop. */
 int pgpu_refine_block(pastix_data_t *pastix_data, int enable);
 
+/* Which kernels the last factorization's FP64 updates took (no counterpart in
+ * the reference): vals[0] = 1 when source column blocks of 32 to 512 columns
+ * went through 8-bit integer slices on the tensor cores, 0 when all updates ran
+ * in FP64 arithmetic (FP32 factors, or digit images that do not fit the device);
+ * vals[1] = LU column blocks that were handed back to FP64 arithmetic because
+ * the slices could not hold their rows (L and U of a row without large entries
+ * in common columns, entries beyond the range of the scales or not finite). */
+int pgpu_get_update_path(const pastix_data_t *pastix_data, pastix_int_t *vals);
+
 /* Bucket boundaries of the supernode update tiles (no counterpart in the
  * reference, whose update GEMM is one BLAS call per blok,
- * kernels/core_zgemmsp.c:404-474).  FP64 factors: an update task whose facing
- * blok has at least dmma_n rows and whose source cblk is at least dmma_k wide
- * runs as 128 x 64 DMMA tiles, any other as 64 x 64 FMA tiles (defaults 32,
+ * kernels/core_zgemmsp.c:404-474).  FP64 factors: tasks with a facing blok of at
+ * least 8 rows and a source cblk 32 to 512 wide run as integer slices (as DMMA
+ * tiles where these cannot be used).  Of the others, a task whose facing blok
+ * has at least dmma_n rows and whose source cblk is at least dmma_k wide
+ * runs as 128 x 64 DMMA tiles, the rest as 64 x 64 FMA tiles (defaults 32,
  * 32).  FP32 factors: a task whose source is at least tc_k (>= 32) wide runs on
  * tcgen05 with split BF16 operands, narrower ones as FMA tiles (default 32).
  * Setting them rebuilds the launch lists: the next pastix_task_numfact /

@@ -89,12 +89,16 @@ void launch_diag_scale(const DevStruct &, int, const T *, T *, int, int, cudaStr
 // update_i8.cu
 long long i8_image_bytes(int, int);
 int i8_max_k();
+template <int F>
 void launch_split_i8(const DevStruct &, const SplitSlab *, int, const double *, const double *, const int64_t *,
-                     unsigned char *, double *, int, cudaStream_t);
+                     unsigned char *, unsigned char *, double *, double *, unsigned long long *, int *, int *, int *,
+                     cudaStream_t);
 template <int F>
 void launch_update_i8(const DevStruct &, const UpdTile *, int, double *, double *, const unsigned char *,
-                      const unsigned char *, const double *, const double *, const int64_t *, int *, int *, bool,
-                      cudaStream_t);
+                      const unsigned char *, const double *, const double *, const int64_t *, const int *, const int *,
+                      int *, int *, bool, cudaStream_t);
+void launch_update_flagged(const DevStruct &, const UpdTile *, int, double *, double *, const int *, const int *,
+                           cudaStream_t);
 cudaError_t set_i8_attrs();
 int sm_count();
 int solve_rows_per_tile();
@@ -190,7 +194,7 @@ struct LevelLists {
     int upds0, upds1;       // k_update tiles (64 x 64), FP32 factors (tasks the tcgen05 kernel does not take)
     int updb0, updb1;       // big update tiles (128 x 64): DMMA for FP64
     int updt0, updt1;       // the same tasks in 128-row aligned windows: tcgen05 for FP32
-    int updm, updbm;        // FP64 lists: tiles from here on belong to tasks that the integer kernel takes
+    int updbm;              // FP64: big tiles from here on belong to tasks that the integer kernel takes
     int upi0, upin, upi1;   // those tasks in 128 x 128 windows (integer slices on tcgen05, FP64 factors): next level's targets, later ones
     int isl0, isl1;         // 128-row slabs of their source cblks, cut into digits
     int updtn, updsn;       // FP32 lists: tiles before these target the next level's cblks
@@ -236,6 +240,8 @@ struct Device {
     DBuf<int64_t> i8_off;
     DBuf<unsigned char> i8_img0, i8_img1;
     DBuf<double> i8_sc0, i8_sc1;
+    DBuf<int> i8_flag;                // LU: sources left to DMMA in the current factorization, by cblk
+    DBuf<unsigned long long> i8_bal;  // LU: column parts of the panels' exponents, two words per column
     bool i8_on = false;      // the images of this factorization fit the device
     // matrix
     DBuf<double> vals, csr_val;
@@ -248,7 +254,7 @@ struct Device {
     DBuf<unsigned char> Lc, Uc, dinv;  // panels; inverted 32x32 diagonal sub-blocks of wide cblks
     int fltsize = 0;
     // work
-    DBuf<int> counters;      // [0] nbpivots, [1] status
+    DBuf<int> counters;      // [0] nbpivots, [1] status, [2] sources flagged by k_split_i8
     DBuf<int> queues;        // tile work-queue heads of the tcgen05 launches, 3 per level, zeroed per factorization
     DBuf<double> dcscr;      // finished panels of the cluster diagonal kernel (read by the cluster's other CTAs)
     DBuf<double> crit;       // [0] static pivoting threshold of the current factorization, [1] ||A||_F
@@ -316,6 +322,7 @@ struct pastix_data_s {
     std::vector<pgpu::SplitSlab> i8_slabs;
     std::vector<int64_t> i8_off;             // byte offset of each cblk's digit image in its level's images (-1: none)
     int64_t i8_total = 0;                    // bytes of the largest level's images (two areas of this size)
+    int i8_used = 0, i8_flagged = 0;         // last factorization: integer updates in use, sources left to DMMA
     std::vector<pgpu::TaskDev> tasks;
     std::vector<int64_t> cb_dinv;
     std::vector<int64_t> sp_off;             // byte offset of each cblk's BF16 image (-1: none)
@@ -1290,24 +1297,21 @@ static int build_maps_and_lists(pastix_data_t *pd) {
         L.upi0 = (int)pd->upd_i8_tiles.size();
         std::vector<pgpu::UpdTile> i8_far;
         L.isl0 = (int)pd->i8_slabs.size();
-        // FP64 tasks of the integer kernel: their DMMA / FMA tiles go to the end of the
-        // lists, where a factorization whose images do not fit the device finds them
+        // FP64 tasks of the integer kernel: their DMMA tiles go to the end of the list, for
+        // flagged sources and for a factorization whose images do not fit the device
         auto i8_task = [&](const pgpu::Task &tk) {
             const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
             return K >= I8_MIN_K && K <= pgpu::i8_max_k() && tk.n >= I8_MIN_N;
         };
         for (int part = 0; part < 2; part++) {
-            if (part) {
-                L.updm = (int)pd->upd_tiles.size();
-                L.updbm = (int)pd->upd_big_tiles.size();
-            }
+            if (part) L.updbm = (int)pd->upd_big_tiles.size();
             for (idx_t t = sv.lvl_task_ptr[l]; t < sv.lvl_task_ptr[l + 1]; t++) {
                 const auto &tk = sv.tasks[t];
                 const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
                 if (K * sv.cb_stride[tk.src] <= SMALL_PANEL_ELEMS) continue;  // done by k_panel_small
                 const bool i8 = i8_task(tk);
                 if (i8 != (part == 1)) continue;
-                const bool big = tk.n >= pd->tune_dmma_n && K >= pd->tune_dmma_k;  // DMMA tiles
+                const bool big = i8 || (tk.n >= pd->tune_dmma_n && K >= pd->tune_dmma_k);  // DMMA tiles
                 const idx_t BM = big ? 128 : 64, BN = 64;
                 auto &list = big ? pd->upd_big_tiles : pd->upd_tiles;
                 for (int side = 0; side < (fk == pgpu::FACT_GETRF ? 2 : 1); side++) {
@@ -1630,6 +1634,10 @@ static int run_factor(pastix_data_t *pd, bool overlap) {
     PdlScope pdl_scope(two && sizeof(T) == 4);
     if (sizeof(T) == 4 || d.i8_on)
         CUDA_TRY(cudaMemsetAsync(d.queues.p, 0, 3 * pd->levels.size() * sizeof(int), st));
+    if (sizeof(T) == 8 && F == pgpu::FACT_GETRF && d.i8_on) {
+        CUDA_TRY(cudaMemsetAsync(d.i8_flag.p, 0, d.i8_flag.n * sizeof(int), st));
+        CUDA_TRY(cudaMemsetAsync(d.i8_bal.p, 0, d.i8_bal.n * sizeof(unsigned long long), st));
+    }
     if (two) {
         CUDA_TRY(cudaEventRecord(d.ev_chain[0], st));
         CUDA_TRY(cudaStreamWaitEvent(d.side, d.ev_chain[0], 0));
@@ -1671,9 +1679,8 @@ static int run_factor(pastix_data_t *pd, bool overlap) {
             });
         }
         if constexpr (sizeof(T) == 8) {
-            const int n = (d.i8_on ? lv.updm : lv.upd1) - lv.upd0;
-            launch_cls(pd, PC_UPDATE, n, [&] {
-                pgpu::launch_update<T, F>(ds, d.upd_tiles.p + lv.upd0, n, L, U, st);
+            launch_cls(pd, PC_UPDATE, lv.upd1 - lv.upd0, [&] {
+                pgpu::launch_update<T, F>(ds, d.upd_tiles.p + lv.upd0, lv.upd1 - lv.upd0, L, U, st);
             });
         } else {
             launch_cls(pd, PC_UPDATE, lv.updsn - lv.upds0, [&] {
@@ -1719,21 +1726,24 @@ static int run_factor(pastix_data_t *pd, bool overlap) {
             });
             if (d.i8_on) {
                 const int nsl = lv.isl1 - lv.isl0;
+                int *lflag = d.queues.p + 3 * l + 1;  // LU: the level has flagged sources
                 launch_cls(pd, PC_SPLIT, nsl, [&] {
-                    const pgpu::SplitSlab *sl = d.i8_slabs.p + lv.isl0;
-                    pgpu::launch_split_i8(ds, sl, nsl, L, L, d.i8_off.p, d.i8_img0.p, d.i8_sc0.p,
-                                          F == pgpu::FACT_POTRF ? 0 : 1, st);
-                    if (F == pgpu::FACT_SYTRF)
-                        pgpu::launch_split_i8(ds, sl, nsl, L, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 2, st);
-                    if (F == pgpu::FACT_GETRF)
-                        pgpu::launch_split_i8(ds, sl, nsl, U, L, d.i8_off.p, d.i8_img1.p, d.i8_sc1.p, 3, st);
+                    pgpu::launch_split_i8<F>(ds, d.i8_slabs.p + lv.isl0, nsl, L, U, d.i8_off.p, d.i8_img0.p, d.i8_img1.p,
+                                             d.i8_sc0.p, d.i8_sc1.p, d.i8_bal.p, d.i8_flag.p, lflag, d.counters.p + 2, st);
                 });
                 const int nnear = (two ? lv.upin : lv.upi1) - lv.upi0;
                 launch_cls(pd, PC_UPDATE_BIG, nnear, [&] {
                     pgpu::launch_update_i8<F>(ds, d.upd_i8_tiles.p + lv.upi0, nnear, L, U, d.i8_img0.p,
-                                              d.i8_img1.p, d.i8_sc0.p, d.i8_sc1.p, d.i8_off.p, d.queues.p + 3 * l,
-                                              d.counters.p + 1, false, st);
+                                              d.i8_img1.p, d.i8_sc0.p, d.i8_sc1.p, d.i8_off.p, d.i8_flag.p, lflag,
+                                              d.queues.p + 3 * l, d.counters.p + 1, false, st);
                 });
+                if (F == pgpu::FACT_GETRF) {
+                    const int nfl = lv.updb1 - lv.updbm;
+                    launch_cls(pd, PC_UPDATE_BIG, nfl, [&] {
+                        pgpu::launch_update_flagged(ds, d.upd_big_tiles.p + lv.updbm, nfl, (double *)L, (double *)U,
+                                                    d.i8_flag.p, lflag, st);
+                    });
+                }
                 if (two) {
                     CUDA_TRY(cudaEventRecord(d.ev_chain[l], st));
                     CUDA_TRY(cudaStreamWaitEvent(d.side, d.ev_chain[l], 0));
@@ -1742,7 +1752,8 @@ static int run_factor(pastix_data_t *pd, bool overlap) {
                         [&] {
                             pgpu::launch_update_i8<F>(ds, d.upd_i8_tiles.p + lv.upin, lv.upi1 - lv.upin, L, U,
                                                       d.i8_img0.p, d.i8_img1.p, d.i8_sc0.p, d.i8_sc1.p, d.i8_off.p,
-                                                      d.queues.p + 3 * l + 2, d.counters.p + 1, true, sd);
+                                                      d.i8_flag.p, lflag, d.queues.p + 3 * l + 2, d.counters.p + 1, true,
+                                                      sd);
                         },
                         sd);
                     CUDA_TRY(cudaEventRecord(d.ev_rest[l], d.side));
@@ -1888,10 +1899,16 @@ extern "C" int pastix_subtask_bcsc2ctab(pastix_data_t *pd) {
     d.i8_on = false;
     if (!pd->mixed && pd->i8_total > 0) {
         const size_t ib = 2 * (size_t)pd->i8_total, nr = pd->solver.rowidx.size();
-        const bool two = fk != pgpu::FACT_POTRF;
+        const bool two = fk != pgpu::FACT_POTRF, lu = fk == pgpu::FACT_GETRF;
         d.i8_on = d.i8_img0.alloc(ib) == cudaSuccess && d.i8_sc0.alloc(nr) == cudaSuccess &&
-                  (!two || (d.i8_img1.alloc(ib) == cudaSuccess && d.i8_sc1.alloc(nr) == cudaSuccess));
+                  (!two || (d.i8_img1.alloc(ib) == cudaSuccess && d.i8_sc1.alloc(nr) == cudaSuccess)) &&
+                  (!lu || (d.i8_flag.alloc(pd->solver.cblknbr) == cudaSuccess &&
+                           d.i8_bal.alloc(2 * (size_t)pd->n) == cudaSuccess));
         if (!d.i8_on) (void)cudaGetLastError();
+    }
+    if (!d.i8_on || fk != pgpu::FACT_GETRF) {
+        d.i8_flag.reset();
+        d.i8_bal.reset();
     }
     if (!d.i8_on || fk == pgpu::FACT_POTRF) {
         d.i8_img1.reset();
@@ -1929,7 +1946,7 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
     // dlamch('e') * ||A|| by default, |magnitude control| when negative, else relative to ||A||
     const double magn = dparm[DPARM_EPSILON_MAGN_CTRL];
     k_threshold<<<1, 1, 0, d.stream>>>(d.crit.p, magn < 0. ? -magn : (magn == 0. ? ldexp(1.0, -53) : magn), magn >= 0.);
-    CUDA_TRY(cudaMemsetAsync(d.counters.p, 0, 2 * sizeof(int), d.stream));
+    CUDA_TRY(cudaMemsetAsync(d.counters.p, 0, 3 * sizeof(int), d.stream));
     CUDA_TRY(cudaEventRecord(d.ev_fact[0], d.stream));
     int fk = fact_kind(pd), rc;
     if (pd->mixed) {
@@ -1955,14 +1972,14 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
         } else {
             const std::vector<uintptr_t> key{1, (uintptr_t)fk, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p,
                                              (uintptr_t)d.i8_img0.p, (uintptr_t)d.i8_img1.p, (uintptr_t)d.i8_sc0.p,
-                                             (uintptr_t)d.i8_sc1.p};
+                                             (uintptr_t)d.i8_sc1.p, (uintptr_t)d.i8_flag.p, (uintptr_t)d.i8_bal.p};
             rc = run_graphed(pd, key, run);
         }
     }
     if (rc) return rc;
-    int cnt[2] = {0, 0};
+    int cnt[3] = {0, 0, 0};
     CUDA_TRY(cudaEventRecord(d.ev_fact[1], d.stream));
-    CUDA_TRY(cudaMemcpyAsync(cnt, d.counters.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, d.stream));
+    CUDA_TRY(cudaMemcpyAsync(cnt, d.counters.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, d.stream));
     rc = fetch_norm(pd);
     if (rc) return rc;
     float ms = 0;
@@ -1973,6 +1990,8 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
     dparm[DPARM_FACT_FLOPS] = t > 0 ? dparm[DPARM_FACT_THFLOPS] / t : 0.0;
     dparm[DPARM_FACT_RLFLOPS] = dparm[DPARM_FACT_THFLOPS];
     pd->iparm[IPARM_STATIC_PIVOTING] = cnt[0];
+    pd->i8_used = d.i8_on;
+    pd->i8_flagged = cnt[2];
     pd->steps |= STEP_NUMFACT;
     return PASTIX_SUCCESS;
 }
@@ -3098,6 +3117,13 @@ extern "C" int pgpu_get_tuning(const pastix_data_t *pd, pastix_int_t *vals) {
     vals[0] = pd->tune_dmma_n;
     vals[1] = pd->tune_dmma_k;
     vals[2] = pd->tune_tc_k;
+    return PASTIX_SUCCESS;
+}
+
+extern "C" int pgpu_get_update_path(const pastix_data_t *pd, pastix_int_t *vals) {
+    if (!pd || !(pd->steps & STEP_NUMFACT) || !vals) return PASTIX_ERR_BADPARAMETER;
+    vals[0] = pd->i8_used;
+    vals[1] = pd->i8_flagged;
     return PASTIX_SUCCESS;
 }
 

@@ -837,8 +837,7 @@ constexpr int DM_LDA = DM_BM + 8, DM_LDB = DM_BN + 8;  // row strides = 8 mod 16
 constexpr size_t DM_SMEM = sizeof(double) * 2 * DM_BK * (DM_LDA + DM_LDB);
 
 template <int FACT>
-__global__ void __launch_bounds__(256) k_update_dmma(DevStruct s, const UpdTile *__restrict__ tiles, double *L,
-                                                      double *U) {
+__device__ __forceinline__ void update_dmma_tile(const DevStruct &s, const UpdTile &tl, double *L, double *U) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *As = reinterpret_cast<double *>(smem_raw);  // [2][DM_BK][DM_LDA]
     double *Bs = As + 2 * DM_BK * DM_LDA;               // [2][DM_BK][DM_LDB]
@@ -846,7 +845,6 @@ __global__ void __launch_bounds__(256) k_update_dmma(DevStruct s, const UpdTile 
     __shared__ int ct[DM_BN];
     __shared__ double dsc[2][DM_BK];
 
-    const UpdTile tl = tiles[blockIdx.x];
     const TaskDev tk = s.tasks[tl.task];
     const int k = tk.src, f = tk.dst;
     const int K = s.cb_lcol[k] - s.cb_fcol[k] + 1;
@@ -968,6 +966,27 @@ __global__ void __launch_bounds__(256) k_update_dmma(DevStruct s, const UpdTile 
             for (int q = 0; q < 8; q++)
                 if (dst[q]) atomicAdd(dst[q], -acc[i][q >> 1][q & 1]);
         }
+    }
+}
+
+template <int FACT>
+__global__ void __launch_bounds__(256) k_update_dmma(DevStruct s, const UpdTile *__restrict__ tiles, double *L,
+                                                      double *U) {
+    update_dmma_tile<FACT>(s, tiles[blockIdx.x], L, U);
+}
+
+// LU: the tiles of the sources that the integer kernel has left (flag, by cblk).
+// The grid strides over the level's `count` tiles and ends at once when the level
+// has no such source.
+__global__ void __launch_bounds__(256) k_update_flagged(DevStruct s, const UpdTile *__restrict__ tiles, int count,
+                                                         double *L, double *U, const int *__restrict__ flag,
+                                                         const int *__restrict__ level_flag) {
+    if (*level_flag == 0) return;
+    for (int t = blockIdx.x; t < count; t += gridDim.x) {
+        const UpdTile tl = tiles[t];
+        if (!flag[s.tasks[tl.task].src]) continue;  // whole CTA
+        update_dmma_tile<FACT_GETRF>(s, tl, L, U);
+        __syncthreads();  // the next tile's tables overwrite this one's
     }
 }
 
@@ -3034,6 +3053,13 @@ void launch_update_big(const DevStruct &s, const UpdTile *tiles, int count, T *L
         k_update<T, FACT, 128, 64, 16, 8, 4><<<count, 256, 0, st>>>(s, tiles, L, U);
 }
 
+// The tiles of a level's flagged sources (LU), on the two CTAs that an SM holds.
+void launch_update_flagged(const DevStruct &s, const UpdTile *tiles, int count, double *L, double *U, const int *flag,
+                           const int *level_flag, cudaStream_t st) {
+    if (count <= 0) return;
+    k_update_flagged<<<std::min(count, 2 * sm_count()), 256, DM_SMEM, st>>>(s, tiles, count, L, U, flag, level_flag);
+}
+
 // CTAs of a persistent update kernel, each of at most `quota` tiles (INT_MAX: one
 // per SM until the tiles are done).  The FP64 updates of far targets run beside the
 // next level's panels on a stream of lower priority; a persistent launch there
@@ -3158,6 +3184,7 @@ cudaError_t set_smem_attrs(size_t, size_t, size_t) {
     }
     if constexpr (sizeof(T) == 8) {
         if ((e = opt_in_smem(k_update_dmma<FACT>)) != cudaSuccess) return e;
+        if (FACT == FACT_GETRF && (e = opt_in_smem(k_update_flagged)) != cudaSuccess) return e;
     } else {
         if ((e = opt_in_smem(k_update_tcp<FACT>)) != cudaSuccess) return e;
         if ((e = opt_in_smem(k_trsm_tcp<FACT>)) != cudaSuccess) return e;

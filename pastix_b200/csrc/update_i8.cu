@@ -24,8 +24,22 @@
 // Rounding relative to the row's largest entry asks for columns of like size:
 // the rows of a Cholesky factor are bounded by the diagonal of A, those of L in
 // LDL^T and LU are not (a small pivot makes a large column).  There column c is
-// scaled by h_c = 2^(half the exponent of the pivot), exactly: (L h)(L D / h)^T
-// and (L h)(U / h), the balance that Cholesky has.
+// scaled by a power of two h_c, exactly: (L h)(L D / h)^T and (L h)(U / h).
+// LDL^T: h_c = 2^(half the exponent of the pivot), the balance that Cholesky has.
+// LU: the pivot does not tell how a scaling of the matrix splits between L and U
+// (scaled rows change L alone by column, scaled columns U alone), so h_c comes
+// from the panels: log2 of their entries is taken as row part + column part, both
+// by least squares (the model of Curtis and Reid, J. Inst. Maths Applics 10,
+// 1972, one sweep, exact for a panel without zeros), and h_c is half of the column
+// part of U less that of L.  Scaling rows or columns of A by powers of two then
+// leaves the digits as they are.  A balance need not exist, so k_split_i8 also
+// checks that every row of L meets its row of U^T: sum_c |l_c u_c| is at least
+// 2^-8 of the product of their largest entries.  That sum is what bounds the FP64
+// rounding of the diagonal entry, about 2^-50.5 of it for 128 columns; 2^-60 a b is
+// then at most 2^-50 of it (LL^T and LDL^T: 2^-58, without a check).  A source with a
+// row that fails, with a row of one factor only, or beyond the range of the scales,
+// is flagged and updated by DMMA instead (launch_update_flagged).  Convection-
+// diffusion on 16 x 15 x 17 to 45 x 38 x 41 points: the smallest ratio is 2^-3.3.
 //
 // Why: the FP64 tensor cores (DMMA) multiply 64 x 2 flops per clock and SM, the
 // 8-bit ones 8192 x 2; 36 digit products per FP64 product are 3.6 times fewer
@@ -57,6 +71,7 @@ constexpr int I8_BN = 128;
 constexpr int I8_TQ = 4;                   // tile-index ring
 constexpr int FAR_TILES_I8 = 6;            // tiles of a CTA of the far updates, about 80 us: 60^3 Laplacian,
                                            // factorization 15.7 -> 13.9 ms against one stream (far_grid)
+constexpr double I8_MEET = 0x1p-8;         // LU: least ratio of sum_c |l_c u_c| to max_c |l_c| max_c |u_c|
 constexpr int I8_MAX_K = 512;              // widest source: the sums i + j >= 4 stay within 2^50
 
 __host__ __device__ inline int i8_nkb(int nc) { return (nc + I8_KB - 1) / I8_KB; }
@@ -68,19 +83,90 @@ long long i8_image_bytes(int nc, int st) { return (long long)I8_S * i8_nkb(nc) *
 int i8_max_k() { return I8_MAX_K; }
 
 // ---------------------------------------------------------------------------
-// Digits of 32-row slabs (blockIdx.y) of 128-row panel slabs.  A lane holds a
-// row; the warps share its 16-column chunks.  The first pass finds the row's
-// largest magnitude, the second (the slab is in L1 / L2 by then) writes the
-// digits, 16 bytes per digit and chunk.  Column factors by `mode`: 0 none, 1 h_c,
-// 2 D_c / h_c, 3 1 / h_c, with D_c the pivot on the diagonal of panel Dp.  Bound
-// by HBM: 8 bytes read and 8 written per entry.
+// LU: the column parts of log2 |entry| in the rows below the diagonal block.
+// blockIdx.z: L or U^T; a lane holds a row, warps share the columns.  Pass one
+// finds each row's mean exponent, pass two (the slab is in L1 / L2 by then) adds
+// the exponents less their row's mean to bal, one word per column and side: the
+// sum in 16ths above 24 bits that count the nonzero entries.  Bound by HBM, the
+// panels of the sources read once more.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *__restrict__ slabs, const double *P,
-                                                  const double *Dp, const int64_t *__restrict__ i8_off,
-                                                  unsigned char *img, double *__restrict__ rscale, int mode) {
-    __shared__ double red[8][32];
+__global__ void __launch_bounds__(256) k_balance_i8(DevStruct s, const SplitSlab *__restrict__ slabs, const double *L,
+                                                    const double *U, unsigned long long *bal) {
+    __shared__ int rsum[8][32], rcnt[8][32];
+    const SplitSlab sl = slabs[blockIdx.x];
+    const int k = sl.cblk;
+    const int nc = s.cb_lcol[k] - s.cb_fcol[k] + 1;
+    const int st = s.cb_stride[k];
+    const int r0 = sl.r0 + 32 * blockIdx.y;
+    if (r0 >= st || r0 + 32 <= nc) return;  // whole CTA
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pr = r0 + lane;
+    const bool in = pr >= nc && pr < st;
+    const double *A = (blockIdx.z ? U : L) + s.cb_coef[k] + pr;
+    auto expo = [&](int c, int (&e)[8]) {  // of columns c, c + 8, ..; 0: zero, subnormal or not finite
+        double v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = (in && c + 8 * j < nc) ? A[(size_t)(c + 8 * j) * st] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            e[j] = (__double2hiint(v[j]) >> 20) & 0x7ff;
+            if (e[j] == 0x7ff) e[j] = 0;
+        }
+    };
+    int sum = 0, cnt = 0;
+    for (int c = warp; c < nc; c += 64) {
+        int e[8];
+        expo(c, e);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            sum += e[j];
+            cnt += e[j] != 0;
+        }
+    }
+    rsum[warp][lane] = sum;
+    rcnt[warp][lane] = cnt;
+    __syncthreads();
+    sum = cnt = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        sum += rsum[w][lane];
+        cnt += rcnt[w][lane];
+    }
+    const int mean = cnt ? 16 * sum / cnt : 0;
+    unsigned long long *dst = bal + 2 * (size_t)s.cb_fcol[k] + blockIdx.z;
+    for (int c = warp; c < nc; c += 64) {
+        int e[8];
+        expo(c, e);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int x = __reduce_add_sync(0xffffffffu, e[j] ? 16 * e[j] - mean : 0);
+            const int num = __popc(__ballot_sync(0xffffffffu, e[j] != 0));
+            if (lane == 0 && num)
+                atomicAdd(dst + 2 * (size_t)(c + 8 * j), (unsigned long long)(x * (1LL << 24) + num));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Digits of 32-row slabs (blockIdx.y) of 128-row panel slabs, of both operands
+// (LDL^T: L h and L D / h; LU: L h and U / h).  A lane holds a row; the warps
+// share its 16-column chunks.  The first pass finds the row's largest magnitudes
+// and for LU the sum_c |l_c u_c|, the second (the slab is in L1 / L2 by then)
+// writes the digits, 16 bytes per digit and chunk.  Bound by HBM: 8 bytes read
+// and 8 written per entry.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double i8_pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
+template <int FACT>
+__global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *__restrict__ slabs, const double *L,
+                                                  const double *U, const int64_t *__restrict__ i8_off,
+                                                  unsigned char *img0, unsigned char *img1, double *__restrict__ sc0,
+                                                  double *__restrict__ sc1, const unsigned long long *__restrict__ bal,
+                                                  int *flag, int *level_flag, int *flagged) {
+    constexpr int SIDES = FACT == FACT_POTRF ? 1 : 2;
+    constexpr bool LU = FACT == FACT_GETRF;
+    __shared__ double red[SIDES][8][32], fsum[LU ? 8 : 1][32];
     __shared__ int badw[8][32];
-    __shared__ double colf[I8_MAX_K];
+    __shared__ double colf[SIDES][I8_MAX_K];
     const SplitSlab sl = slabs[blockIdx.x];
     const int k = sl.cblk;
     const int nc = s.cb_lcol[k] - s.cb_fcol[k] + 1;
@@ -89,95 +175,139 @@ __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *
     const int pr = sl.r0 + 32 * blockIdx.y + lane;
     if (sl.r0 + 32 * (int)blockIdx.y >= st) return;  // whole CTA
     const int nkb = i8_nkb(nc), ng = i8_ng(st), nch = 2 * nkb;
-    const double *A = P + s.cb_coef[k] + pr;
-    const double *D = Dp + s.cb_coef[k];
-    auto load = [&](int ch, double (&v)[16]) {
+    const double *AL = L + s.cb_coef[k] + pr, *AU = LU ? U + s.cb_coef[k] + pr : AL;
+    auto load = [&](int side, int ch, double (&v)[16]) {
+        const double *A = side ? AU : AL;
 #pragma unroll
         for (int j = 0; j < 16; j++) {
             const int c = 16 * ch + j;
             v[j] = (pr < st && c < nc) ? A[(size_t)c * st] : 0.0;
         }
-        if (mode) {
+        if (FACT != FACT_POTRF) {
 #pragma unroll
             for (int j = 0; j < 16; j++) {
                 const int c = 16 * ch + j;
-                if (c < nc) v[j] *= colf[c];
+                if (c < nc) v[j] *= colf[side][c];
             }
         }
     };
-    auto pow2 = [](int e) { return __hiloint2double((e + 1023) << 20, 0); };
-    if (mode) {
+    if (FACT == FACT_SYTRF) {
         for (int c = threadIdx.x; c < nc; c += 256) {
-            const double d = D[c + (size_t)c * st];
+            const double d = L[s.cb_coef[k] + c + (size_t)c * st];
             const int e = (__double2hiint(d) >> 20) & 0x7ff;
             const int h = (e == 0 || e == 0x7ff) ? 0 : (e - 1023) / 2;  // zero and non-finite pivots: none
-            colf[c] = mode == 1 ? pow2(h) : (mode == 2 ? d * pow2(-h) : pow2(-h));
+            colf[0][c] = i8_pow2(h);
+            colf[SIDES - 1][c] = d * i8_pow2(-h);
         }
         __syncthreads();
     }
-    double m = 0.0;
+    if (LU) {
+        for (int c = threadIdx.x; c < nc; c += 256) {
+            const long long bl = (long long)bal[2 * (size_t)(s.cb_fcol[k] + c)];
+            const long long bu = (long long)bal[2 * (size_t)(s.cb_fcol[k] + c) + 1];
+            const int nl = (int)(bl & 0xffffff), nu = (int)(bu & 0xffffff);
+            int h = 0;  // a column without entries on one side: none
+            if (nl && nu) h = __float2int_rn(((float)(bu >> 24) / (float)nu - (float)(bl >> 24) / (float)nl) * 0x1p-5f);
+            h = max(-1000, min(1000, h));
+            colf[0][c] = i8_pow2(h);
+            colf[SIDES - 1][c] = i8_pow2(-h);
+        }
+        __syncthreads();
+    }
+    double m[SIDES], f = 0.0;
     int bad = 0;
+#pragma unroll
+    for (int q = 0; q < SIDES; q++) m[q] = 0.0;
     for (int ch = warp; ch < nch; ch += 8) {
-        double v[16];
-        load(ch, v);
+        double v[SIDES][16];
+#pragma unroll
+        for (int q = 0; q < SIDES; q++) load(q, ch, v[q]);
 #pragma unroll
         for (int j = 0; j < 16; j++) {
-            const double a = fabs(v[j]);
-            m = a > m ? a : m;
-            bad |= !(a <= 1.7976931348623157e308);
+#pragma unroll
+            for (int q = 0; q < SIDES; q++) {
+                const double a = fabs(v[q][j]);
+                m[q] = a > m[q] ? a : m[q];
+                bad |= !(a <= 1.7976931348623157e308) << q;
+            }
+            if (LU) f += fabs(v[0][j] * v[SIDES - 1][j]);
         }
     }
-    red[warp][lane] = m;
+#pragma unroll
+    for (int q = 0; q < SIDES; q++) red[q][warp][lane] = m[q];
     badw[warp][lane] = bad;
+    if (LU) fsum[warp][lane] = f;
     __syncthreads();
+    f = 0.0;
 #pragma unroll
     for (int w = 0; w < 8; w++) {
-        m = red[w][lane] > m ? red[w][lane] : m;
+#pragma unroll
+        for (int q = 0; q < SIDES; q++) m[q] = red[q][w][lane] > m[q] ? red[q][w][lane] : m[q];
         bad |= badw[w][lane];
+        if (LU) f += fsum[w][lane];
     }
-    // row exponent: |a| < 127.375 / 128 * 2^ex, so that the leading digit fits 8
-    // bits after the carries of the balanced digits (at most 0.502 of it)
-    const int mhi = __double2hiint(m);
-    int ex = ((mhi >> 20) & 0x7ff) - 1022;
-    if ((mhi & 0xfffff) >= 0xfd800) ex++;  // mantissa of 2 * 127.375 / 128
-    if (ex < -958) ex = -958;              // smaller rows: rounded at 2^-1021, as subnormal numbers are
-    const double mult = bad ? 0.0 : pow2(I8_BITS - ex);
-    if (warp == 0 && pr < st)
-        rscale[s.cb_rowidx[k] + pr] = bad ? __longlong_as_double(0x7ff8000000000000LL) : pow2(ex - 19);
-    if (pr >= 8 * ((st + 7) / 8)) return;
-    unsigned char *out = img + i8_off[k] + (size_t)(pr >> 3) * I8_GROUP + (pr & 7) * 16;
-    for (int ch = warp; ch < nch; ch += 8) {
-        double v[16];
-        load(ch, v);
-        uint32_t w[I8_S][4];
-#pragma unroll
-        for (int g = 0; g < 4; g++) {
-            uint32_t lo[4], hi[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const long long q = bad ? 0 : __double2ll_rn(v[4 * g + j] * mult);
-                const unsigned long long t = (unsigned long long)q + 0x80808080808080ULL;
-                lo[j] = (uint32_t)t;
-                hi[j] = (uint32_t)(t >> 32);
-            }
-            // byte b of the four values, by 4 x 4 byte transposes
-            const uint32_t l01a = __byte_perm(lo[0], lo[1], 0x5140), l23a = __byte_perm(lo[2], lo[3], 0x5140);
-            const uint32_t l01b = __byte_perm(lo[0], lo[1], 0x7362), l23b = __byte_perm(lo[2], lo[3], 0x7362);
-            const uint32_t h01a = __byte_perm(hi[0], hi[1], 0x5140), h23a = __byte_perm(hi[2], hi[3], 0x5140);
-            const uint32_t h01b = __byte_perm(hi[0], hi[1], 0x7362), h23b = __byte_perm(hi[2], hi[3], 0x7362);
-            w[7][g] = __byte_perm(l01a, l23a, 0x5410) ^ 0x80808080u;
-            w[6][g] = __byte_perm(l01a, l23a, 0x7632) ^ 0x80808080u;
-            w[5][g] = __byte_perm(l01b, l23b, 0x5410) ^ 0x80808080u;
-            w[4][g] = __byte_perm(l01b, l23b, 0x7632) ^ 0x80808080u;
-            w[3][g] = __byte_perm(h01a, h23a, 0x5410) ^ 0x80808080u;
-            w[2][g] = __byte_perm(h01a, h23a, 0x7632) ^ 0x80808080u;
-            w[1][g] = __byte_perm(h01b, h23b, 0x5410) ^ 0x80808080u;
-            w[0][g] = __byte_perm(h01b, h23b, 0x7632);
+    if (LU && warp == 0) {
+        // rows that the integer products cannot take: see the head of this file.  A
+        // scaled entry that left the range of FP64 is among them (bad), and so is a
+        // source with a non-finite entry, which DMMA carries on.
+        const double ab = m[0] * m[SIDES - 1];
+        const bool off = pr >= nc && pr < st;
+        const bool fails = bad || (m[0] > 0.0) != (m[SIDES - 1] > 0.0) ||
+                           (m[0] > 0.0 && !(ab >= 0x1p-1000 && f <= 0x1p1000 && f >= I8_MEET * ab &&
+                                            m[0] >= 0x1p-950 && m[SIDES - 1] >= 0x1p-950));
+        if (__any_sync(0xffffffffu, off && fails) && lane == 0) {
+            *level_flag = 1;
+            if (atomicExch(flag + k, 1) == 0) atomicAdd(flagged, 1);
         }
-        unsigned char *o = out + (size_t)(ch >> 1) * ng * I8_GROUP + (ch & 1) * 128;
+    }
 #pragma unroll
-        for (int p = 0; p < I8_S; p++)
-            *reinterpret_cast<uint4 *>(o + (size_t)p * nkb * ng * I8_GROUP) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    for (int q = 0; q < SIDES; q++) {
+        // row exponent: |a| < 127.375 / 128 * 2^ex, so that the leading digit fits 8
+        // bits after the carries of the balanced digits (at most 0.502 of it)
+        const bool nan = (bad >> q) & 1;
+        const int mhi = __double2hiint(m[q]);
+        int ex = ((mhi >> 20) & 0x7ff) - 1022;
+        if ((mhi & 0xfffff) >= 0xfd800) ex++;  // mantissa of 2 * 127.375 / 128
+        if (ex < -958) ex = -958;              // smaller rows: rounded at 2^-1021, as subnormal numbers are
+        const double mult = nan ? 0.0 : i8_pow2(I8_BITS - ex);
+        if (warp == 0 && pr < st)
+            (q ? sc1 : sc0)[s.cb_rowidx[k] + pr] = nan ? __longlong_as_double(0x7ff8000000000000LL) : i8_pow2(ex - 19);
+        if (pr >= 8 * ((st + 7) / 8)) continue;
+        unsigned char *out = (q ? img1 : img0) + i8_off[k] + (size_t)(pr >> 3) * I8_GROUP + (pr & 7) * 16;
+        for (int ch = warp; ch < nch; ch += 8) {
+            double v[16];
+            load(q, ch, v);
+            uint32_t w[I8_S][4];
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                uint32_t lo[4], hi[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const long long i = nan ? 0 : __double2ll_rn(v[4 * g + j] * mult);
+                    const unsigned long long t = (unsigned long long)i + 0x80808080808080ULL;
+                    lo[j] = (uint32_t)t;
+                    hi[j] = (uint32_t)(t >> 32);
+                }
+                // byte b of the four values, by 4 x 4 byte transposes
+                const uint32_t l01a = __byte_perm(lo[0], lo[1], 0x5140), l23a = __byte_perm(lo[2], lo[3], 0x5140);
+                const uint32_t l01b = __byte_perm(lo[0], lo[1], 0x7362), l23b = __byte_perm(lo[2], lo[3], 0x7362);
+                const uint32_t h01a = __byte_perm(hi[0], hi[1], 0x5140), h23a = __byte_perm(hi[2], hi[3], 0x5140);
+                const uint32_t h01b = __byte_perm(hi[0], hi[1], 0x7362), h23b = __byte_perm(hi[2], hi[3], 0x7362);
+                w[7][g] = __byte_perm(l01a, l23a, 0x5410) ^ 0x80808080u;
+                w[6][g] = __byte_perm(l01a, l23a, 0x7632) ^ 0x80808080u;
+                w[5][g] = __byte_perm(l01b, l23b, 0x5410) ^ 0x80808080u;
+                w[4][g] = __byte_perm(l01b, l23b, 0x7632) ^ 0x80808080u;
+                w[3][g] = __byte_perm(h01a, h23a, 0x5410) ^ 0x80808080u;
+                w[2][g] = __byte_perm(h01a, h23a, 0x7632) ^ 0x80808080u;
+                w[1][g] = __byte_perm(h01b, h23b, 0x5410) ^ 0x80808080u;
+                w[0][g] = __byte_perm(h01b, h23b, 0x7632);
+            }
+            unsigned char *o = out + (size_t)(ch >> 1) * ng * I8_GROUP + (ch & 1) * 128;
+#pragma unroll
+            for (int p = 0; p < I8_S; p++)
+                *reinterpret_cast<uint4 *>(o + (size_t)p * nkb * ng * I8_GROUP) =
+                    make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+        }
     }
 }
 
@@ -242,7 +372,8 @@ template <int FACT>
 __global__ void __launch_bounds__(I8_THREADS, 1)
     k_update_i8(DevStruct s, const UpdTile *__restrict__ tiles, int count, int quota, double *L, double *U,
                 const unsigned char *img0, const unsigned char *img1, const double *__restrict__ sc0,
-                const double *__restrict__ sc1, const int64_t *__restrict__ i8_off, int *queue, int *status) {
+                const double *__restrict__ sc1, const int64_t *__restrict__ i8_off, const int *flag,
+                const int *level_flag, int *queue, int *status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[I8_STAGES], empty[I8_STAGES], tfull, tempty, tq_full[I8_TQ], tq_empty[I8_TQ];
     __shared__ uint32_t tmem_sh;
@@ -278,14 +409,18 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
         if (lane == 0) {  // producer: claims tiles, loads their operands
             uint32_t g = 0;
             int next = atomicAdd(queue, 1);  // claimed one tile ahead
+            // LU: tiles of flagged sources are left to DMMA
+            const bool any = FACT == FACT_GETRF && *level_flag != 0;
+            auto skipped = [&](int t) { return any && t < count && flag[s.tasks[tiles[t].task].src] != 0; };
             for (int j = 0; !late; j++) {
                 const int slot = j % I8_TQ;
                 if (j >= I8_TQ && !mbar_wait(&tq_empty[slot], ((j / I8_TQ) - 1) & 1)) {
                     late = 1;
                     break;
                 }
-                int t = next;
-                if (t >= count || j >= quota) t = -1;  // `quota`: tiles of this CTA
+                int t = j < quota ? next : count;  // `quota`: tiles of this CTA
+                while (skipped(t)) t = atomicAdd(queue, 1);
+                if (t >= count) t = -1;
                 else if (j + 1 < quota) next = atomicAdd(queue, 1);
                 tq[slot] = t;
                 mbar_arrive(&tq_full[slot]);
@@ -479,19 +614,24 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
-void launch_split_i8(const DevStruct &s, const SplitSlab *slabs, int count, const double *P, const double *D,
-                     const int64_t *i8_off, unsigned char *img, double *rscale, int scale, cudaStream_t st) {
+template <int FACT>
+void launch_split_i8(const DevStruct &s, const SplitSlab *slabs, int count, const double *L, const double *U,
+                     const int64_t *i8_off, unsigned char *img0, unsigned char *img1, double *sc0, double *sc1,
+                     unsigned long long *bal, int *flag, int *level_flag, int *flagged, cudaStream_t st) {
     if (count <= 0) return;
-    k_split_i8<<<dim3(count, 4), 256, 0, st>>>(s, slabs, P, D, i8_off, img, rscale, scale);
+    if (FACT == FACT_GETRF) k_balance_i8<<<dim3(count, 4, 2), 256, 0, st>>>(s, slabs, L, U, bal);
+    k_split_i8<FACT><<<dim3(count, 4), 256, 0, st>>>(s, slabs, L, U, i8_off, img0, img1, sc0, sc1, bal, flag, level_flag,
+                                                     flagged);
 }
 template <int FACT>
 void launch_update_i8(const DevStruct &s, const UpdTile *tiles, int count, double *L, double *U,
                       const unsigned char *img0, const unsigned char *img1, const double *sc0, const double *sc1,
-                      const int64_t *i8_off, int *queue, int *status, bool far, cudaStream_t st) {
+                      const int64_t *i8_off, const int *flag, const int *level_flag, int *queue, int *status, bool far,
+                      cudaStream_t st) {
     if (count <= 0) return;
     const int quota = far ? FAR_TILES_I8 : INT_MAX;
     k_update_i8<FACT><<<far_grid(count, quota), I8_THREADS, I8_SMEM, st>>>(s, tiles, count, quota, L, U, img0, img1, sc0,
-                                                                           sc1, i8_off, queue, status);
+                                                                           sc1, i8_off, flag, level_flag, queue, status);
 }
 cudaError_t set_i8_attrs() {
     cudaError_t e = cudaSuccess;
@@ -500,9 +640,12 @@ cudaError_t set_i8_attrs() {
     return e;
 }
 #define PGPU_INST_I8(F)                                                                                               \
+    template void launch_split_i8<F>(const DevStruct &, const SplitSlab *, int, const double *, const double *,       \
+                                     const int64_t *, unsigned char *, unsigned char *, double *, double *,           \
+                                     unsigned long long *, int *, int *, int *, cudaStream_t);                        \
     template void launch_update_i8<F>(const DevStruct &, const UpdTile *, int, double *, double *,                    \
                                       const unsigned char *, const unsigned char *, const double *, const double *,   \
-                                      const int64_t *, int *, int *, bool, cudaStream_t);
+                                      const int64_t *, const int *, const int *, int *, int *, bool, cudaStream_t);
 PGPU_INST_I8(FACT_POTRF)
 PGPU_INST_I8(FACT_SYTRF)
 PGPU_INST_I8(FACT_GETRF)

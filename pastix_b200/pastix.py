@@ -373,6 +373,13 @@ def get_tuning(pd: Data) -> tuple:
     return tuple(int(x) for x in v)
 
 
+def get_update_path(pd: Data) -> tuple:
+    """(integer slices used, LU column blocks handed back to FP64 arithmetic) of the last factorization."""
+    v = np.zeros(2, dtype=np.int64)
+    _check("pgpu_get_update_path", _lib.load().pgpu_get_update_path(pd.ptr, v.ctypes.data_as(PINT)))
+    return bool(v[0]), int(v[1])
+
+
 def autotune(pd: Data, values) -> tuple:
     """Time the candidate update-tile buckets on factorizations of `values` (CUDA
     float64 tensor, spm order); the fastest stays in effect.  Returns
