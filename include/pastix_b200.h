@@ -379,10 +379,15 @@ int pgpu_graphs(pastix_data_t *pastix_data, int enable);
  * simple refinement keep the column loop. */
 int pgpu_refine_block(pastix_data_t *pastix_data, int enable);
 
+/* FP64 updates by integer slices on the tensor cores (default on).  enable = 0:
+ * the next factorizations form every FP64 update in FP64 arithmetic. */
+int pgpu_integer_updates(pastix_data_t *pastix_data, int enable);
+
 /* Which kernels the last factorization's FP64 updates took (no counterpart in
  * the reference): vals[0] = 1 when source column blocks of 32 to 512 columns
  * went through 8-bit integer slices on the tensor cores, 0 when all updates ran
- * in FP64 arithmetic (FP32 factors, or digit images that do not fit the device);
+ * in FP64 arithmetic (FP32 factors, switched off, or digit images that do not fit
+ * the device);
  * vals[1] = LU column blocks that were handed back to FP64 arithmetic because
  * the slices could not hold their rows (L and U of a row without large entries
  * in common columns, entries beyond the range of the scales or not finite). */

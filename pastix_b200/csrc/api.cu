@@ -322,6 +322,7 @@ struct pastix_data_s {
     std::vector<pgpu::SplitSlab> i8_slabs;
     std::vector<int64_t> i8_off;             // byte offset of each cblk's digit image in its level's images (-1: none)
     int64_t i8_total = 0;                    // bytes of the largest level's images (two areas of this size)
+    bool i8_enable = true;                   // pgpu_integer_updates
     int i8_used = 0, i8_flagged = 0;         // last factorization: integer updates in use, sources left to DMMA
     std::vector<pgpu::TaskDev> tasks;
     std::vector<int64_t> cb_dinv;
@@ -1897,7 +1898,7 @@ extern "C" int pastix_subtask_bcsc2ctab(pastix_data_t *pd) {
     }
     // FP64: digit images of one level's panels; a factorization for which they do not fit runs on DMMA
     d.i8_on = false;
-    if (!pd->mixed && pd->i8_total > 0) {
+    if (!pd->mixed && pd->i8_enable && pd->i8_total > 0) {
         const size_t ib = 2 * (size_t)pd->i8_total, nr = pd->solver.rowidx.size();
         const bool two = fk != pgpu::FACT_POTRF, lu = fk == pgpu::FACT_GETRF;
         d.i8_on = d.i8_img0.alloc(ib) == cudaSuccess && d.i8_sc0.alloc(nr) == cudaSuccess &&
@@ -3117,6 +3118,12 @@ extern "C" int pgpu_get_tuning(const pastix_data_t *pd, pastix_int_t *vals) {
     vals[0] = pd->tune_dmma_n;
     vals[1] = pd->tune_dmma_k;
     vals[2] = pd->tune_tc_k;
+    return PASTIX_SUCCESS;
+}
+
+extern "C" int pgpu_integer_updates(pastix_data_t *pd, int enable) {
+    if (!pd) return PASTIX_ERR_BADPARAMETER;
+    pd->i8_enable = enable != 0;
     return PASTIX_SUCCESS;
 }
 

@@ -373,6 +373,11 @@ def get_tuning(pd: Data) -> tuple:
     return tuple(int(x) for x in v)
 
 
+def integer_updates(pd: Data, enable: bool) -> None:
+    """FP64 updates by integer slices (default on); off: the next factorizations stay in FP64 arithmetic."""
+    _check("pgpu_integer_updates", _lib.load().pgpu_integer_updates(pd.ptr, int(enable)))
+
+
 def get_update_path(pd: Data) -> tuple:
     """(integer slices used, LU column blocks handed back to FP64 arithmetic) of the last factorization."""
     v = np.zeros(2, dtype=np.int64)

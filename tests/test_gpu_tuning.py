@@ -72,6 +72,25 @@ def test_buckets_give_same_factors(lib, fact, mixed):
     assert lib.pgpu_device_status(pd.ptr) == 0
 
 
+@pytest.mark.parametrize("fact", ["POTRF", "SYTRF", "GETRF"])
+def test_buckets_without_integer_updates(lib, fact):
+    """FP64 arithmetic for every task, back and forth with the integer slices in one handle."""
+    A, grid = _case(fact)
+    pd, S, info = analyse(A, grid, fact)
+    vals = torch.tensor(S.values, device="cuda")
+    keep = _used(info, fact)
+    ref, npiv0 = _factors(pd, vals, fact, keep)
+    assert px.get_update_path(pd) == (True, 0)
+    for st in ((32, 32, 32), (8, 16, 32), (1, 1, 32), (64, 32, 32)):
+        px.set_tuning(pd, *st)
+        for integer in (False, True):
+            px.integer_updates(pd, integer)
+            got, npiv = _factors(pd, vals, fact, keep)
+            assert px.get_update_path(pd) == (integer, 0) and npiv == npiv0
+            for g, r in zip(got, ref):
+                assert _rel(g, r) <= TOL[False], (st, integer, _rel(g, r))
+
+
 @pytest.mark.parametrize("mixed", [False, True])
 def test_autotune(lib, mixed):
     A, grid = _case("POTRF")

@@ -30,9 +30,22 @@ def _system(fact):
 @pytest.mark.parametrize("fact", ["POTRF", "SYTRF", "GETRF"])
 @pytest.mark.parametrize("bs", [(32, 33), (40, 64), (64, 65), (96, 129), (160, 320)])
 def test_factors_at_tile_edges(lib, oracle_mod, fact, bs):
+    _factors_against_oracle(oracle_mod, fact, bs, True)
+
+
+@pytest.mark.parametrize("fact", ["POTRF", "SYTRF", "GETRF"])
+@pytest.mark.parametrize("bs", [(32, 33), (40, 64), (64, 65), (160, 320)])
+def test_fp64_tiles_of_the_same_tasks(lib, oracle_mod, fact, bs):
+    """The DMMA tiles that take these tasks where the integer slices cannot be used."""
+    _factors_against_oracle(oracle_mod, fact, bs, False)
+
+
+def _factors_against_oracle(oracle_mod, fact, bs, integer):
     A, grid = _system(fact)
     pd, S, info = analyse(A, grid, fact, min_bs=bs[0], max_bs=bs[1])
+    px.integer_updates(pd, integer)
     px.task_numfact(pd, S)
+    assert px.get_update_path(pd) == (integer, 0)
     Lg, Ug = px.get_coeftab(pd, with_u=(fact == "GETRF"))
     sym = oracle_mod.Symbol(info)
     Ap = oracle_mod.permuted_full(S.full(), info["permtab"])
