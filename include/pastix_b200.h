@@ -387,7 +387,9 @@ int pgpu_integer_updates(pastix_data_t *pastix_data, int enable);
  * the reference): vals[0] = 1 when source column blocks of 32 to 512 columns
  * went through 8-bit integer slices on the tensor cores, 0 when all updates ran
  * in FP64 arithmetic (FP32 factors, switched off, or digit images that do not fit
- * the device);
+ * the device with 512 MiB and 64 vectors left free: checked once per analysis or
+ * pgpu_integer_updates call.  The images are given back when a later allocation
+ * of the handle finds no other memory);
  * vals[1] = LU column blocks that were handed back to FP64 arithmetic because
  * the slices could not hold their rows (L and U of a row without large entries
  * in common columns, entries beyond the range of the scales or not finite). */

@@ -158,6 +158,9 @@ namespace {
 // integer-slice tiles, the others DMMA or FMA tiles: a K block is 32 columns and
 // the least N of a tile 16, so that below these lines most of a product is padding.
 constexpr idx_t I8_MIN_K = 32, I8_MIN_N = 8;
+// Device memory left free beside their images, with 64 vectors of the matrix on top:
+// a restarted GMRES of 25 steps and a solve of several right-hand sides.
+constexpr size_t I8_RESERVE = 512u << 20;
 constexpr idx_t SMALL_PANEL_ELEMS = 4096;  // st*nc below which a cblk is factored in one CTA's smem
 
 template <typename X>
@@ -242,7 +245,21 @@ struct Device {
     DBuf<double> i8_sc0, i8_sc1;
     DBuf<int> i8_flag;                // LU: sources left to DMMA in the current factorization, by cblk
     DBuf<unsigned long long> i8_bal;  // LU: column parts of the panels' exponents, two words per column
-    bool i8_on = false;      // the images of this factorization fit the device
+    bool i8_on = false;      // this factorization uses them
+    bool i8_nofit = false;   // they did not fit beside the rest, or were given back to it
+    // Gives the images' memory back: they serve one factorization's updates, and
+    // whatever else a handle allocates goes first.
+    bool release_images() {
+        const bool held = i8_img0.p || i8_img1.p;
+        i8_on = false;
+        i8_img0.reset();
+        i8_img1.reset();
+        i8_sc0.reset();
+        i8_sc1.reset();
+        i8_flag.reset();
+        i8_bal.reset();
+        return held;
+    }
     // matrix
     DBuf<double> vals, csr_val;
     DBuf<int64_t> lmap, umap, csr_src, perm;
@@ -380,11 +397,35 @@ static inline void launch_cls(pastix_data_t *pd, int cls, long long count, Fn &&
 enum : int { WS_SOLVE = 0, WS_ORDER, WS_GMV, WS_GMW, WS_GMG, WS_VEC, WS_BP, WS_XP, WS_RB, WS_RX, WS_BGV, WS_BGS,
              WS_SPSV, WS_GMH };
 
+// Allocation that takes the memory of the digit images when there is no other left.
+static cudaError_t dev_malloc(Device &d, void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && d.release_images()) {
+        (void)cudaGetLastError();
+        d.i8_nofit = true;
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+template <typename X>
+static cudaError_t grow(Device &d, DBuf<X> &b, size_t count) {
+    if (count == b.n && b.p) return cudaSuccess;
+    b.reset();
+    if (count == 0) return cudaSuccess;
+    void *p = nullptr;
+    const cudaError_t e = dev_malloc(d, &p, count * sizeof(X));
+    if (e == cudaSuccess) {
+        b.p = (X *)p;
+        b.n = count;
+    }
+    return e;
+}
+
 // Persistent device work area `slot` of at least `count` doubles (grown, never shrunk).
 static double *work(Device &d, int slot, size_t count) {
     DBuf<double> &b = d.ws[slot];
     if (b.n < count) {
-        if (b.alloc(count) != cudaSuccess) return nullptr;
+        if (grow(d, b, count) != cudaSuccess) return nullptr;
     }
     return b.p;
 }
@@ -1492,6 +1533,8 @@ static int device_setup(pastix_data_t *pd) {
     if (d.ready) { CUDA_TRY(cudaSetDevice(d.dev)); return PASTIX_SUCCESS; }
     if (d.stream) CUDA_TRY(cudaStreamSynchronize(d.stream));
     pd->graphs.clear();  // captured launches name the old structure
+    d.release_images();
+    d.i8_nofit = false;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         perr("no CUDA device available: the numerical phase runs on the GPU only");
@@ -1863,6 +1906,12 @@ extern "C" int pastix_subtask_bcsc2ctab(pastix_data_t *pd) {
     const int fs = pd->mixed ? 4 : 8;
     const int fk = fact_kind(pd);
     const size_t bytes = (size_t)std::max<idx_t>(1, pd->solver.coefnbr) * fs;
+    const size_t i8_bytes = 2 * (size_t)pd->i8_total;
+    const bool i8_want = !pd->mixed && pd->i8_enable && i8_bytes > 0 && !d.i8_nofit;
+    // images that this factorization has no use for go before anything is allocated
+    if (!i8_want || d.i8_img0.n != i8_bytes || d.Lc.n != bytes || (fk != pgpu::FACT_POTRF) != (d.i8_img1.p != nullptr) ||
+        (fk == pgpu::FACT_GETRF) != (d.i8_flag.p != nullptr))
+        d.release_images();
     if (d.Lc.n != bytes) CUDA_TRY(d.Lc.alloc(bytes));
     if (fk == pgpu::FACT_GETRF) { if (d.Uc.n != bytes) CUDA_TRY(d.Uc.alloc(bytes)); }
     else d.Uc.reset();
@@ -1896,28 +1945,27 @@ extern "C" int pastix_subtask_bcsc2ctab(pastix_data_t *pd) {
         d.tinv.reset();
         d.timg.reset();
     }
-    // FP64: digit images of one level's panels; a factorization for which they do not fit runs on DMMA
-    d.i8_on = false;
-    if (!pd->mixed && pd->i8_enable && pd->i8_total > 0) {
-        const size_t ib = 2 * (size_t)pd->i8_total, nr = pd->solver.rowidx.size();
+    // FP64: digit images of two levels' panels.  A factorization for which they do
+    // not fit, with room left for what the solves and the refinement allocate later,
+    // runs on DMMA; that is remembered until the lists are rebuilt or
+    // pgpu_integer_updates is called, so that it is not tried on every call.
+    if (i8_want && d.i8_img0.n == i8_bytes) {
+        d.i8_on = true;
+    } else if (i8_want) {
+        const size_t nr = pd->solver.rowidx.size(), n = (size_t)pd->n;
         const bool two = fk != pgpu::FACT_POTRF, lu = fk == pgpu::FACT_GETRF;
-        d.i8_on = d.i8_img0.alloc(ib) == cudaSuccess && d.i8_sc0.alloc(nr) == cudaSuccess &&
-                  (!two || (d.i8_img1.alloc(ib) == cudaSuccess && d.i8_sc1.alloc(nr) == cudaSuccess)) &&
-                  (!lu || (d.i8_flag.alloc(pd->solver.cblknbr) == cudaSuccess &&
-                           d.i8_bal.alloc(2 * (size_t)pd->n) == cudaSuccess));
-        if (!d.i8_on) (void)cudaGetLastError();
-    }
-    if (!d.i8_on || fk != pgpu::FACT_GETRF) {
-        d.i8_flag.reset();
-        d.i8_bal.reset();
-    }
-    if (!d.i8_on || fk == pgpu::FACT_POTRF) {
-        d.i8_img1.reset();
-        d.i8_sc1.reset();
-    }
-    if (!d.i8_on) {
-        d.i8_img0.reset();
-        d.i8_sc0.reset();
+        const size_t need = (two ? 2 : 1) * (i8_bytes + 8 * nr) + (lu ? 16 * n + 4 * (size_t)pd->solver.cblknbr : 0);
+        size_t fr = 0, tot = 0;
+        CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+        d.i8_on = fr >= need + I8_RESERVE + 64 * 8 * n && d.i8_img0.alloc(i8_bytes) == cudaSuccess &&
+                  d.i8_sc0.alloc(nr) == cudaSuccess &&
+                  (!two || (d.i8_img1.alloc(i8_bytes) == cudaSuccess && d.i8_sc1.alloc(nr) == cudaSuccess)) &&
+                  (!lu || (d.i8_flag.alloc(pd->solver.cblknbr) == cudaSuccess && d.i8_bal.alloc(2 * n) == cudaSuccess));
+        if (!d.i8_on) {
+            (void)cudaGetLastError();
+            d.release_images();
+            d.i8_nofit = true;
+        }
     }
     CUDA_TRY(cudaMemsetAsync(d.Lc.p, 0, bytes, d.stream));
     if (d.Uc.p) CUDA_TRY(cudaMemsetAsync(d.Uc.p, 0, bytes, d.stream));
@@ -2141,7 +2189,7 @@ static int solve_perm_d(pastix_data_t *pd, int trans, double *Y, int ldy, int nr
         });
     }
     size_t need = (size_t)pd->n * nrhs;
-    if (d.wf.n < need) CUDA_TRY(d.wf.alloc(need));
+    if (d.wf.n < need) CUDA_TRY(grow(d, d.wf, need));
     const std::vector<uintptr_t> key{2, 1, (uintptr_t)trans, (uintptr_t)fact_kind(pd), (uintptr_t)Y, (uintptr_t)ldy,
                                      (uintptr_t)nrhs, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p,
                                      (uintptr_t)d.tinv.p, (uintptr_t)d.wf.p};
@@ -2170,7 +2218,7 @@ static int solve_device_orig(pastix_data_t *pd, int trans, int nrhs, double *B, 
     CUDA_TRY(cudaSetDevice(d.dev));
     const idx_t n = pd->n;
     size_t need = (size_t)n * nrhs;
-    if (d.w1.n < need) CUDA_TRY(d.w1.alloc(need));
+    if (d.w1.n < need) CUDA_TRY(grow(d, d.w1, need));
     cudaEvent_t ev = nullptr;
     if (user != d.stream) {  // order the library stream after the caller's (NULL = legacy default) stream
         CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -2242,11 +2290,12 @@ extern "C" int pastixRhsFinalize(pastix_rhs_t rhs) {
     free(rhs);
     return PASTIX_SUCCESS;
 }
-static int rhs_alloc(pastix_rhs_t r, int flt, pastix_int_t m, pastix_int_t n) {
+static int rhs_alloc(Device *d, pastix_rhs_t r, int flt, pastix_int_t m, pastix_int_t n) {
     size_t es = flt == SpmFloat ? 4 : 8;
     if (r->allocated && r->b) cudaFree(r->b);
     r->b = nullptr;
-    CUDA_TRY(cudaMalloc(&r->b, std::max<size_t>(1, (size_t)m * n) * es));
+    const size_t bytes = std::max<size_t>(1, (size_t)m * n) * es;
+    CUDA_TRY(d ? dev_malloc(*d, &r->b, bytes) : cudaMalloc(&r->b, bytes));
     r->allocated = 1;
     r->flttype = flt;
     r->m = m;
@@ -2256,7 +2305,7 @@ static int rhs_alloc(pastix_rhs_t r, int flt, pastix_int_t m, pastix_int_t n) {
 }
 extern "C" int pastixRhsDoubletoSingle(const pastix_rhs_t dB, pastix_rhs_t sB) {
     if (!dB || !sB || dB->flttype != SpmDouble) return PASTIX_ERR_BADPARAMETER;
-    int rc = rhs_alloc(sB, SpmFloat, dB->m, dB->n);
+    int rc = rhs_alloc(nullptr, sB, SpmFloat, dB->m, dB->n);
     if (rc) return rc;
     for (pastix_int_t j = 0; j < dB->n; j++)
         pgpu::launch_cast<double, float>(dB->m, (const double *)dB->b + j * dB->ld, (float *)sB->b + j * sB->ld, 0);
@@ -2283,7 +2332,7 @@ extern "C" int pastix_subtask_applyorder(pastix_data_t *pd, pastix_dir_t dir, pa
     if (!tmp) return PASTIX_ERR_OUTOFMEMORY;
     if (dir == PastixDirForward) {
         if (!(Bp->b && Bp->m == m && Bp->n == n && Bp->flttype == SpmDouble)) {
-            rc = rhs_alloc(Bp, SpmDouble, m, n);
+            rc = rhs_alloc(&d, Bp, SpmDouble, m, n);
             if (rc) return rc;
         }
         CUDA_TRY(cudaMemcpy2DAsync(tmp, m * 8, B, ldb * 8, m * 8, n, cudaMemcpyHostToDevice, d.stream));
@@ -2978,8 +3027,8 @@ extern "C" int pgpu_spmv_device(pastix_data_t *pd, double alpha, const double *x
         return PASTIX_SUCCESS;
     }
     // y overlaps x: through permuted copies
-    if (d.w1.n < (size_t)pd->n) CUDA_TRY(d.w1.alloc(pd->n));
-    if (d.w2.n < (size_t)pd->n) CUDA_TRY(d.w2.alloc(pd->n));
+    if (d.w1.n < (size_t)pd->n) CUDA_TRY(grow(d, d.w1, pd->n));
+    if (d.w2.n < (size_t)pd->n) CUDA_TRY(grow(d, d.w2, pd->n));
     CUDA_TRY(cudaStreamSynchronize(d.stream));  // the work vectors are shared with the library stream
     pgpu::launch_permute<double, double>((int)pd->n, 1, d.perm.p, 1, x, pd->n, d.w1.p, pd->n, st);
     pgpu::launch_permute<double, double>((int)pd->n, 1, d.perm.p, 1, y, pd->n, d.w2.p, pd->n, st);
@@ -3124,6 +3173,7 @@ extern "C" int pgpu_get_tuning(const pastix_data_t *pd, pastix_int_t *vals) {
 extern "C" int pgpu_integer_updates(pastix_data_t *pd, int enable) {
     if (!pd) return PASTIX_ERR_BADPARAMETER;
     pd->i8_enable = enable != 0;
+    pd->dev.i8_nofit = false;
     return PASTIX_SUCCESS;
 }
 
