@@ -179,6 +179,7 @@ struct DBuf {  // owning device buffer
         if (cnt == 0) return cudaSuccess;
         cudaError_t e = cudaMalloc(&p, cnt * sizeof(X));
         if (e == cudaSuccess) n = cnt;
+        else (void)cudaGetLastError();  // returned here; the next call's check must not find it
         return e;
     }
     cudaError_t upload(const std::vector<X> &v, cudaStream_t st) {
@@ -405,6 +406,7 @@ static cudaError_t dev_malloc(Device &d, void **p, size_t bytes) {
         d.i8_nofit = true;
         e = cudaMalloc(p, bytes);
     }
+    if (e != cudaSuccess) (void)cudaGetLastError();
     return e;
 }
 template <typename X>
@@ -2045,21 +2047,26 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
     return PASTIX_SUCCESS;
 }
 
+// Panels and factors from values that are on their way to the device.  A call that
+// fails returns once they and their norm are in place, as one that succeeds does:
+// products (pgpu_spmv_device) read them from other streams, and the caller may
+// reuse its array.
+static int factor_values(pastix_data_t *pd) {
+    int rc = pastix_subtask_bcsc2ctab(pd);
+    if (!rc) rc = pastix_subtask_sopalin(pd);
+    if (rc) (void)fetch_norm(pd);
+    return rc;
+}
+
 extern "C" int pastix_task_numfact(pastix_data_t *pd, spmatrix_t *spm) {
     int rc = spm2bcsc_host(pd, spm);
-    if (rc) return rc;
-    rc = pastix_subtask_bcsc2ctab(pd);
-    if (rc) return rc;
-    return pastix_subtask_sopalin(pd);
+    return rc ? rc : factor_values(pd);
 }
 
 extern "C" int pgpu_numfact_device(pastix_data_t *pd, const double *values_dev) {
     if (!pd || !values_dev) return PASTIX_ERR_BADPARAMETER;
     int rc = spm2bcsc_common(pd, values_dev, true, SpmDouble);
-    if (rc) return rc;
-    rc = pastix_subtask_bcsc2ctab(pd);
-    if (rc) return rc;
-    return pastix_subtask_sopalin(pd);
+    return rc ? rc : factor_values(pd);
 }
 
 extern "C" int pgpu_get_coeftab(const pastix_data_t *pd, void *L, void *U) {

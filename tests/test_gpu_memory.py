@@ -89,3 +89,26 @@ def test_images_are_given_back(lib, fact):
     assert px.get_update_path(pd) == (False, 0)
     assert _solves(pd, S, 3)
     px.finalize(pd)
+
+
+def test_failed_factorization_leaves_the_values_in_place(lib):
+    """Panels that cannot be allocated: the call fails after the values were taken.  They and their norm are complete
+    when it returns, and a product on another stream sees them."""
+    pd, S, v = _handle("POTRF")
+    pd.iparm[px.iparm.mixed] = 1
+    px.numfact_device(pd, v)
+    pd.iparm[px.iparm.mixed] = 0  # panels of twice the size
+    w = 2.0 * v
+    pd.dparm[px.dparm.a_norm] = 0.0
+    with _filled(8 * MIB), pytest.raises(px.PastixError):
+        px.numfact_device(pd, w)
+    norm = float(pd.dparm[px.dparm.a_norm])
+    A = 2.0 * S.full()
+    assert abs(norm - np.sqrt((A.data ** 2).sum())) < 1e-12 * norm
+    x = torch.rand(S.n, dtype=torch.float64, device="cuda")
+    y = torch.zeros_like(x)
+    px.spmv_device(pd, 1.0, x, 0.0, y)
+    assert np.linalg.norm(y.cpu().numpy() - A @ x.cpu().numpy()) < 1e-13 * np.linalg.norm(y.cpu().numpy())
+    px.numfact_device(pd, w)
+    assert px.get_update_path(pd) == (True, 0)
+    px.finalize(pd)
