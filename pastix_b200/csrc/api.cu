@@ -1081,6 +1081,12 @@ extern "C" int pastix_subtask_reordering(pastix_data_t *pd) {
     return PASTIX_SUCCESS;
 }
 
+// FP64 update tasks of the integer kernel.
+static bool i8_task(const pgpu::Solver &sv, const pgpu::Task &tk) {
+    const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
+    return K >= I8_MIN_K && K <= pgpu::i8_max_k() && tk.n >= I8_MIN_N;
+}
+
 // Host-side construction of the value maps and of the launch lists.
 static int build_maps_and_lists(pastix_data_t *pd) {
     const pgpu::Solver &sv = pd->solver;
@@ -1343,17 +1349,13 @@ static int build_maps_and_lists(pastix_data_t *pd) {
         L.isl0 = (int)pd->i8_slabs.size();
         // FP64 tasks of the integer kernel: their DMMA tiles go to the end of the list, for
         // flagged sources and for a factorization whose images do not fit the device
-        auto i8_task = [&](const pgpu::Task &tk) {
-            const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
-            return K >= I8_MIN_K && K <= pgpu::i8_max_k() && tk.n >= I8_MIN_N;
-        };
         for (int part = 0; part < 2; part++) {
             if (part) L.updbm = (int)pd->upd_big_tiles.size();
             for (idx_t t = sv.lvl_task_ptr[l]; t < sv.lvl_task_ptr[l + 1]; t++) {
                 const auto &tk = sv.tasks[t];
                 const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
                 if (K * sv.cb_stride[tk.src] <= SMALL_PANEL_ELEMS) continue;  // done by k_panel_small
-                const bool i8 = i8_task(tk);
+                const bool i8 = i8_task(sv, tk);
                 if (i8 != (part == 1)) continue;
                 const bool big = i8 || (tk.n >= pd->tune_dmma_n && K >= pd->tune_dmma_k);  // DMMA tiles
                 const idx_t BM = big ? 128 : 64, BN = 64;
@@ -3202,6 +3204,7 @@ extern "C" int pgpu_autotune(pastix_data_t *pd, const double *values_dev, pastix
         return PASTIX_ERR_BADPARAMETER;
     }
     pd->mixed = pd->iparm[IPARM_MIXED] ? 1 : 0;
+    const auto &sv = pd->solver;
     std::vector<std::array<int, 3>> cands;
     if (pd->mixed) {
         for (int tk : {32, 48, 64, 96}) cands.push_back({pd->tune_dmma_n, pd->tune_dmma_k, tk});
@@ -3214,6 +3217,23 @@ extern "C" int pgpu_autotune(pastix_data_t *pd, const double *values_dev, pastix
     const std::array<int, 3> cur{pd->tune_dmma_n, pd->tune_dmma_k, pd->tune_tc_k};
     cands.erase(std::remove(cands.begin(), cands.end(), cur), cands.end());
     cands.insert(cands.begin(), cur);
+    if (!pd->mixed) {
+        // the integer slices take most tasks whatever the buckets say: of the candidates that
+        // sort the rest alike only the first is timed
+        std::vector<std::vector<char>> sorted;
+        auto seen = [&](const std::array<int, 3> &c) {
+            std::vector<char> big;
+            for (const auto &tk : sv.tasks) {
+                const idx_t K = sv.cb_lcol[tk.src] - sv.cb_fcol[tk.src] + 1;
+                if (K * sv.cb_stride[tk.src] > SMALL_PANEL_ELEMS && !i8_task(sv, tk))
+                    big.push_back(tk.n >= c[0] && K >= c[1]);
+            }
+            if (std::find(sorted.begin(), sorted.end(), big) != sorted.end()) return true;
+            sorted.push_back(std::move(big));
+            return false;
+        };
+        cands.erase(std::remove_if(cands.begin(), cands.end(), seen), cands.end());
+    }
     double best = 1e300;
     std::array<int, 3> arg = cur;
     for (const auto &c : cands) {

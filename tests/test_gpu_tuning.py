@@ -91,6 +91,26 @@ def test_buckets_without_integer_updates(lib, fact):
                 assert _rel(g, r) <= TOL[False], (st, integer, _rel(g, r))
 
 
+def test_autotune_times_each_sorting_once(lib):
+    """FP64 buckets that sort the tasks outside the integer slices alike are one candidate."""
+    A, grid = _case("POTRF")
+    pd, S, info = analyse(A, grid, "POTRF")
+    nc = info["cb_lcol"] - info["cb_fcol"] + 1
+    tasks = []  # (blok height, source width)
+    for k in range(int(info["cblknbr"])):
+        if nc[k] * info["cb_stride"][k] > 4096:
+            b = np.arange(info["cb_fblok"][k] + 1, info["cb_fblok"][k + 1])
+            tasks += [(int(n), int(nc[k])) for n in info["bk_lrow"][b] - info["bk_frow"][b] + 1]
+    rest = [(n, K) for n, K in tasks if K < 32 or K > 512 or n < 8]
+    sortings = {tuple(n >= cn and K >= ck for n, K in rest) for cn in (8, 16, 32, 64) for ck in (16, 32)}
+    assert len(sortings) < 8
+    vals = torch.tensor(S.values, device="cuda")
+    px.profile(pd, False)
+    px.autotune(pd, vals)
+    # three factorizations for each, one more with the choice
+    assert px.profile_get(pd)["fill"][1] == 3 * len(sortings) + 1
+
+
 @pytest.mark.parametrize("mixed", [False, True])
 def test_autotune(lib, mixed):
     A, grid = _case("POTRF")
