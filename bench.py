@@ -122,7 +122,7 @@ def max_over_ranks(t: float, ws: int, device: str = "cuda") -> float:
 
 
 def fp64_peak_tflops(torch) -> float:
-    """cuBLAS DGEMM throughput measured in this run (the FP64 roofline denominator)."""
+    """cuBLAS DGEMM throughput measured in this run."""
     n = 8192
     a = torch.randn(n, n, dtype=torch.float64, device="cuda")
     b = torch.randn(n, n, dtype=torch.float64, device="cuda")
@@ -330,6 +330,14 @@ def run_b200(args, ws, rank, local):
             results[mode]["d2h"] = 8 * n + 8 * n
         px.finalize(pd)
     return results, n
+
+
+def reference_missing() -> str | None:
+    """Why the reference cannot be run on this machine, None if it can."""
+    from oracle import ref
+    if ref.available():
+        return None
+    return "the library built from the reference's sources (oracle/_ref) is not on this machine"
 
 
 def run_reference(args, modes=("mixed", "fp64"), nsteps: int = 1, warmup: int = 0) -> dict:
@@ -633,6 +641,10 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return 0
+        why = reference_missing()
+        if why:
+            print(json.dumps({"impl": "reference", "unavailable": why}))
+            return 0
         # a full-workload step takes tens of seconds on the host cores: at most
         # two per mode, so that the whole run stays within a few minutes
         r = run_reference(args, nsteps=max(1, min(args.steps, 2)), warmup=1)
@@ -656,10 +668,11 @@ def main():
     value = res[best]["t"]
     prof = fp64["profile"]
     uflops = update_flops(fp64["info"])
-    # FP64 path: update GEMMs (integer slices on tcgen05, DMMA) against the cuBLAS DGEMM rate measured here
+    # FP64 path: update GEMMs as integer slices on tcgen05, 36 8-bit products (twice the bf16 rate) per FP64 product;
+    # the cuBLAS DGEMM rate measured here is reported beside it
     upd_ms = prof["update"][0] + prof["update_big"][0]
     upd_launch = prof["update"][1] + prof["update_big"][1]
-    peak64 = fp64_peak_tflops(torch) if rank == 0 else None
+    dgemm = fp64_peak_tflops(torch) if rank == 0 else None
     ach64 = uflops / (upd_ms / 1e3) / 1e12 if upd_ms > 0 else None
     # FP32 path (the headline when it wins): tcgen05 update GEMMs, six BF16 products per FP32 product
     prof32 = mixed["profile"]
@@ -674,6 +687,9 @@ def main():
     bf16 = peaks.get("bf16_tflops")
     peak32 = bf16 / 6.0 if bf16 else 1590.0 / 6.0
     ach32 = uflops / (tc_ms / 1e3) / 1e12 if tc_ms > 0 else None
+    peak64 = 2.0 * (bf16 or 1590.0) / 36.0
+    peak64_src = ("measured dense bf16 %s TFLOP/s (MEASURED_PEAKS.json, burst) x 2 / 36 8-bit products per FP64 product"
+                  % bf16) if bf16 else "fallback 1590 TFLOP/s bf16 x 2 / 36"
     traffic = None
     tfile = ROOT / "profiles" / "traffic.json"
     if tfile.exists():
@@ -691,8 +707,8 @@ def main():
     else:
         roof = {"kernel": "k_update_i8 + k_update_dmma + k_update (FP64 supernode update GEMMs + scatter-add)", "bound": "tensor",
                 "achieved": ach64, "peak": peak64, "unit": "TFLOP/s",
-                "frac": (ach64 / peak64) if (ach64 and peak64) else None, "traffic": None,
-                "peak_source": "cuBLAS DGEMM 8192^3 measured in this run", "launches": upd_launch,
+                "frac": (ach64 / peak64) if ach64 else None, "traffic": None,
+                "peak_source": peak64_src, "launches": upd_launch,
                 "ms_total": upd_ms, "algorithmic_flops": uflops}
     line = {
         "metric": metric, "value": value, "unit": "s", "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
@@ -710,8 +726,8 @@ def main():
         "static_pivots": fp64["npiv"],
         "roofline": roof,
         "roofline_fp64": {"kernel": "k_update_i8 + k_update_dmma + k_update", "achieved": ach64, "peak": peak64,
-                          "unit": "TFLOP/s", "frac": (ach64 / peak64) if (ach64 and peak64) else None,
-                          "peak_source": "cuBLAS DGEMM 8192^3 measured in this run"},
+                          "unit": "TFLOP/s", "frac": (ach64 / peak64) if ach64 else None, "peak_source": peak64_src,
+                          "dgemm": dgemm, "dgemm_source": "cuBLAS DGEMM 8192^3 measured in this run"},
         "profile_ms": {k: v[0] for k, v in prof.items() if v[1]},
         "profile_ms_fp32": {k: v[0] for k, v in mixed["profile"].items() if v[1]},
         "clocks": mixed["clocks"],
@@ -733,9 +749,14 @@ def main():
         line["adjoint"] = run_adjoint()
     if rank == 0 and not args.no_cpu_baseline and ws == 1:
         # one step of the reference's faster mode (FP32 factors + FP64 CG) on the full workload
-        cb = run_reference(args, modes=("mixed",), nsteps=1)
-        line["cpu_baseline"] = {"value": cb["t"], "unit": "s", "cores": cb["threads"], "kind": "reference",
-                                "sample": reference_sample(cb, WORKLOADS[args.workload][0])}
+        why = reference_missing()
+        if why:
+            line["cpu_baseline"] = None
+            line["cpu_baseline_unavailable"] = why
+        else:
+            cb = run_reference(args, modes=("mixed",), nsteps=1)
+            line["cpu_baseline"] = {"value": cb["t"], "unit": "s", "cores": cb["threads"], "kind": "reference",
+                                    "sample": reference_sample(cb, WORKLOADS[args.workload][0])}
     if rank == 0:
         print(json.dumps(line))
     if ws > 1:

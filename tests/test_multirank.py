@@ -1,9 +1,10 @@
 """Host logic of multi-GPU runs, on CPU with two gloo ranks: bench.py's
 replicas report the slowest rank's time on every rank, and the ranks other
 than 0 of the reference arm exit without output (rank 0 alone runs and prints
-the CPU baseline)."""
+the CPU baseline); the arm's line where the reference is not built."""
 from __future__ import annotations
 
+import json
 import os
 import socket
 import subprocess
@@ -54,3 +55,16 @@ def test_reference_arm_other_ranks_exit_quietly():
                        env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0
     assert r.stdout.strip() == ""
+
+
+def test_reference_arm_without_the_reference(monkeypatch, capsys):
+    """A machine without the library built from the reference's sources: one line that says so, exit code 0."""
+    import bench
+    from oracle import ref
+    monkeypatch.setattr(ref, "LIB", ROOT / "oracle" / "_ref" / "absent.so")
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference"])
+    for k in ("RANK", "WORLD_SIZE", "LOCAL_RANK"):
+        monkeypatch.delenv(k, raising=False)
+    assert bench.main() == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"]
