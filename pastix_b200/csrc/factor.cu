@@ -2661,6 +2661,7 @@ __device__ __forceinline__ void tc_persistent(int count, int *queue, int *status
                                               ColInfo colinfo, Epi epi) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[TP_STAGES], empty[TP_STAGES], tfull[2], tempty[2], tq_full[TQ], tq_empty[TQ];
+    __shared__ __align__(8) uint64_t drained;
     __shared__ uint32_t tmem_sh;
     __shared__ int ctab[2][TC_BN];
     __shared__ int tq[TQ];
@@ -2683,6 +2684,7 @@ __device__ __forceinline__ void tc_persistent(int count, int *queue, int *status
             mbar_init(&tq_full[i], 1);
             mbar_init(&tq_empty[i], 1 + 4 * 32);  // the MMA issuer and the 128 epilogue threads
         }
+        mbar_init(&drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     tc_fence_before();
@@ -2690,9 +2692,9 @@ __device__ __forceinline__ void tc_persistent(int count, int *queue, int *status
     tc_fence_after();
     const uint32_t tmem = tmem_sh;
     int late = 0;
+    uint32_t g = 0;  // producer, MMA issuer: K blocks so far
     if (warp == 4) {
         if (lane == 0) {  // producer: claims tiles, loads their operands
-            uint32_t g = 0;
             // the claim of the next tile is issued one tile ahead, so that its
             // round trip to L2 overlaps this tile's copies
             int next = atomicAdd(queue, 1);
@@ -2732,7 +2734,6 @@ __device__ __forceinline__ void tc_persistent(int count, int *queue, int *status
     } else if (warp == 5) {
         if (lane == 0) {  // MMA issuer
             const uint32_t sbase = smem_u32(smem_raw);
-            uint32_t g = 0;
             for (int i = 0; !late; i++) {
                 const int slot = i % TQ;
                 if (!mbar_wait(&tq_full[slot], (i / TQ) & 1)) {
@@ -2811,7 +2812,12 @@ __device__ __forceinline__ void tc_persistent(int count, int *queue, int *status
     }
     __syncwarp();
     const int aborted = __syncthreads_or(late);
-    if (aborted && tid == 0) atomicExch(status, PGPU_STATUS_TIMEOUT);
+    if (aborted) {  // nothing of this CTA may be in flight when it ends
+        if (tid == 0) atomicExch(status, PGPU_STATUS_TIMEOUT);
+        if (warp == 4 && lane == 0) drain_loads(full, TP_STAGES, g);
+        if (warp == 5 && lane == 0) drain_mmas(&drained);
+        __syncthreads();
+    }
     tc_fence_after();
     if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TC_BN));
 }
@@ -3118,33 +3124,52 @@ int trinv_max_blocks() { return DG_MAXNC / 32; }
 // k_diag_cluster does, on a flag of CTA 0 that nothing raises, while CTA 0
 // waits, as the tcgen05 engine does, on an mbarrier phase that nothing
 // completes.  Both waits give up; timed_out[r] counts CTA r's, and the kernel
-// ends with the context usable.
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32) k_wait_selftest(int *timed_out) {
+// ends with the context usable.  CTA 0 has bulk copies of `src` (64 bytes) in flight
+// meanwhile, three loads into a ring of two, which it waits for as the engine does.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32) k_wait_selftest(int *timed_out, const int *src) {
     namespace cg = cooperative_groups;
     __shared__ int flag;
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bar, full[2];
+    __shared__ __align__(16) int ring[2][16];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     if (threadIdx.x == 0) {
         flag = 0;
         mbar_init(&bar, 1);
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cluster.sync();
     if (threadIdx.x == 0) {
+        bool landed = true;
+        if (rank == 0) {
+            for (int g = 0; g < 3; g++) {
+                if (g == 2) landed &= mbar_wait(&full[0], 0);  // the ring's first buffer is free again
+                mbar_expect_tx(&full[g & 1], 64);
+                bulk_g2s(ring[g & 1], src, 64, &full[g & 1]);
+            }
+        }
         const bool ok = (rank == 1) ? dc_wait(dsmem_map(&flag, 0), 1) : mbar_wait(&bar, 0);
-        if (!ok) atomicAdd(timed_out + rank, 1);
+        if (rank == 0) {
+            landed &= drain_loads(full, 2, 3);
+            for (int i = 0; i < 32; i++) landed &= ring[i >> 4][i & 15] == 7;
+        }
+        if (!ok) atomicAdd(timed_out + rank, landed ? 1 : 2);
     }
     cluster.sync();  // CTA 0's shared memory outlives CTA 1's reads
 }
 cudaError_t wait_selftest(int *timed_out_host) {
-    int *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, 2 * sizeof(int));
+    int *d = nullptr;  // 16 sevens, then the two counters
+    int init[18];
+    std::fill(init, init + 16, 7);
+    init[16] = init[17] = 0;
+    cudaError_t e = cudaMalloc(&d, sizeof(init));
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemset(d, 0, 2 * sizeof(int))) == cudaSuccess) {
-        k_wait_selftest<<<2, 32>>>(d);
+    if ((e = cudaMemcpy(d, init, sizeof(init), cudaMemcpyHostToDevice)) == cudaSuccess) {
+        k_wait_selftest<<<2, 32>>>(d + 16, d);
         if ((e = cudaGetLastError()) == cudaSuccess && (e = cudaDeviceSynchronize()) == cudaSuccess)
-            e = cudaMemcpy(timed_out_host, d, 2 * sizeof(int), cudaMemcpyDeviceToHost);
+            e = cudaMemcpy(timed_out_host, d + 16, 2 * sizeof(int), cudaMemcpyDeviceToHost);
     }
     cudaFree(d);
     return e;

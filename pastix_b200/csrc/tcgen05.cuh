@@ -48,5 +48,19 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// Ahead of a CTA's early end, once a wait has given up: the bulk copies that the
+// calling thread has issued into a ring of `stages` buffers (`issued` loads so far,
+// each completing a phase of its stage's full[]) are waited for, bounded too, and
+// so are the MMAs that it has issued (through `bar`, not used before).
+__device__ __forceinline__ bool drain_loads(uint64_t *full, uint32_t stages, uint32_t issued) {
+    bool ok = true;
+    for (uint32_t i = issued > stages ? issued - stages : 0; i < issued; i++)
+        ok &= mbar_wait(&full[i % stages], (i / stages) & 1);
+    return ok;
+}
+__device__ __forceinline__ bool drain_mmas(uint64_t *bar) {
+    tc_commit(bar);
+    return mbar_wait(bar, 0);
+}
 
 }  // namespace pgpu

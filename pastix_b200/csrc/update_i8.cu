@@ -376,6 +376,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
                 const int *level_flag, int *queue, int *status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[I8_STAGES], empty[I8_STAGES], tfull, tempty, tq_full[I8_TQ], tq_empty[I8_TQ];
+    __shared__ __align__(8) uint64_t drained;
     __shared__ uint32_t tmem_sh;
     __shared__ int ctab[2][I8_BN];
     __shared__ double csc[2][I8_BN];
@@ -394,6 +395,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
         }
         mbar_init(&tfull, 1);
         mbar_init(&tempty, I8_EPI);
+        mbar_init(&drained, 1);
         for (int i = 0; i < I8_TQ; i++) {
             mbar_init(&tq_full[i], 1);
             mbar_init(&tq_empty[i], 1 + I8_EPI);
@@ -405,9 +407,9 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_sh;
     int late = 0;
+    uint32_t g = 0;  // producer, MMA issuer: K blocks so far
     if (warp == 8) {
         if (lane == 0) {  // producer: claims tiles, loads their operands
-            uint32_t g = 0;
             int next = atomicAdd(queue, 1);  // claimed one tile ahead
             // LU: tiles of flagged sources are left to DMMA
             const bool any = FACT == FACT_GETRF && *level_flag != 0;
@@ -459,7 +461,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
     } else if (warp == 9) {
         if (lane == 0) {  // MMA issuer
             const uint32_t sbase = smem_u32(smem_raw);
-            uint32_t g = 0, ph = 0;
+            uint32_t ph = 0;
             for (int i = 0; !late; i++) {
                 const int slot = i % I8_TQ;
                 if (!mbar_wait(&tq_full[slot], (i / I8_TQ) & 1)) {
@@ -608,7 +610,12 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
     }
     __syncwarp();
     const int aborted = __syncthreads_or(late);
-    if (aborted && tid == 0) atomicExch(status, PGPU_STATUS_TIMEOUT);
+    if (aborted) {  // nothing of this CTA may be in flight when it ends
+        if (tid == 0) atomicExch(status, PGPU_STATUS_TIMEOUT);
+        if (warp == 8 && lane == 0) drain_loads(full, I8_STAGES, g);
+        if (warp == 9 && lane == 0) drain_mmas(&drained);
+        __syncthreads();
+    }
     tc_fence_after();
     if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(4 * I8_BN));
 }
