@@ -2973,7 +2973,11 @@ void launch_panel_small(const DevStruct &s, const int *list, int count, size_t s
 }
 
 // 16-CTA clusters of the LU kernel that the current device runs at once (0: none), for a
-// launch with `smem` dynamic bytes per CTA.
+// launch with `smem` dynamic bytes per CTA.  A level with more such blocks takes one
+// CTA per block (k_diag_dmma).  72^3 convection-diffusion, us, clusters | one CTA each:
+// two waves of clusters 8 blocks 575..620 | 790..950, 10 blocks 600 | 905..945; three
+// or four waves 16 blocks 840..890 | 795..860, 24 blocks (64^3) 990 | 570.  One wave
+// (7 blocks 375) is well on the clusters' side of the line, which lies behind two.
 template <typename T>
 static int dc16_clusters(size_t smem) {
     cudaLaunchConfig_t cfg = {};

@@ -966,9 +966,12 @@ __global__ void k_diag_scale(DevStruct s, const T *L, T *Y, int ldy, int nrhs) {
 // ------------------------------ launchers ---------------------------------
 // Whether the diagonal kernels of a level's `count` narrow cblks apply their rows
 // too: one right-hand side, and enough cblks that a warp each fills the SMs.
-// Levels of few, larger cblks take longer that way than two launches (512^2
-// diffusion, FP64: 64 cblks 26 us forward and 28 backward against about 10; 2048
-// and more 11 and 25 against 20 and 30).
+// The warp against the diagonal kernel and the update launch, FP64, us, forward and
+// backward: 512^2 grid 512 cblks 10.7 | 13.2 and 11.0 | 12.1, 1024 8.1 | 13.2 and
+// 10.8 | 13.3, 2048 6.4 | 15.9 and 9.4 | 18.8, 16385 35 | 85 and 53 | 123; 80^3
+// Laplacian 2030 larger ones 19 | 38 and 30 | 46; 64 of the 512^2 grid's, larger
+// still, 26 | 10 and 28 | 10.  The line lies at the smallest count that is clearly
+// ahead both ways.
 bool solve_fuse_rows(int count, int nrhs) { return nrhs == 1 && count >= 1024; }
 // One right-hand side or groups of 8 (a group's missing columns are masked).
 template <typename T>
