@@ -391,8 +391,9 @@ int pgpu_integer_updates(pastix_data_t *pastix_data, int enable);
  * pgpu_integer_updates call.  The images are given back when a later allocation
  * of the handle finds no other memory);
  * vals[1] = LU column blocks that were handed back to FP64 arithmetic because
- * the slices could not hold their rows (L and U of a row without large entries
- * in common columns, entries beyond the range of the scales or not finite). */
+ * the slices would lose digits there: rows of L or U that are large against the
+ * diagonal, as when rows or columns of the matrix are scaled on one side only, or
+ * entries beyond the range of the scales or not finite. */
 int pgpu_get_update_path(const pastix_data_t *pastix_data, pastix_int_t *vals);
 
 /* Bucket boundaries of the supernode update tiles (no counterpart in the

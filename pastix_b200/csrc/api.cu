@@ -91,8 +91,8 @@ long long i8_image_bytes(int, int);
 int i8_max_k();
 template <int F>
 void launch_split_i8(const DevStruct &, const SplitSlab *, int, const double *, const double *, const int64_t *,
-                     unsigned char *, unsigned char *, double *, double *, unsigned long long *, int *, int *, int *,
-                     cudaStream_t);
+                     unsigned char *, unsigned char *, double *, double *, const double *, const int *, int *, int *,
+                     int *, cudaStream_t);
 template <int F>
 void launch_update_i8(const DevStruct &, const UpdTile *, int, double *, double *, const unsigned char *,
                       const unsigned char *, const double *, const double *, const int64_t *, const int *, const int *,
@@ -245,7 +245,6 @@ struct Device {
     DBuf<unsigned char> i8_img0, i8_img1;
     DBuf<double> i8_sc0, i8_sc1;
     DBuf<int> i8_flag;                // LU: sources left to DMMA in the current factorization, by cblk
-    DBuf<unsigned long long> i8_bal;  // LU: column parts of the panels' exponents, two words per column
     bool i8_on = false;      // this factorization uses them
     bool i8_nofit = false;   // they did not fit beside the rest, or were given back to it
     // Gives the images' memory back: they serve one factorization's updates, and
@@ -258,7 +257,6 @@ struct Device {
         i8_sc0.reset();
         i8_sc1.reset();
         i8_flag.reset();
-        i8_bal.reset();
         return held;
     }
     // matrix
@@ -267,6 +265,7 @@ struct Device {
     DBuf<int> csr_rowptr, csr_col, e_row, e_col;
     DBuf<int> csr_colo, peri;  // columns in the caller's numbering, matrix row of every permuted row
     DBuf<int> spmv_part;     // row blocks of the streamed SpMV
+    DBuf<int> csr_diag;      // LU: entry of the CSR on the diagonal of every permuted row (-1: none)
     int spmv_nblocks = 0;
     // factor
     DBuf<unsigned char> Lc, Uc, dinv;  // panels; inverted 32x32 diagonal sub-blocks of wide cblks
@@ -331,6 +330,7 @@ struct pastix_data_s {
     // value maps (host, structure only)
     std::vector<int64_t> lmap, umap, csr_src;
     std::vector<int> csr_rowptr, csr_col, e_row, e_col;
+    std::vector<int> csr_diag;
     idx_t csr_nnz = 0;
     std::vector<LevelLists> levels;
     // host copies of the launch lists
@@ -1181,6 +1181,15 @@ static int build_maps_and_lists(pastix_data_t *pd) {
             }
         }
     }
+    pd->csr_diag.clear();
+    if (fk == pgpu::FACT_GETRF) {
+        pd->csr_diag.assign(n, -1);
+        for (idx_t i = 0; i < n; i++) {
+            const auto b = pd->csr_col.begin() + pd->csr_rowptr[i], e = pd->csr_col.begin() + pd->csr_rowptr[i + 1];
+            const auto it = std::lower_bound(b, e, (int)i);
+            if (it != e && *it == (int)i) pd->csr_diag[i] = (int)(it - pd->csr_col.begin());
+        }
+    }
 
     // ---- launch lists per level ----
     pd->levels.assign(sv.nlevels, LevelLists{});
@@ -1608,6 +1617,7 @@ static int device_setup(pastix_data_t *pd) {
         CUDA_TRY(d.spmv_part.upload(part, st));
     }
     CUDA_TRY(d.csr_col.upload(pd->csr_col, st));
+    CUDA_TRY(d.csr_diag.upload(pd->csr_diag, st));
     CUDA_TRY(d.e_row.upload(pd->e_row, st));
     CUDA_TRY(d.e_col.upload(pd->e_col, st));
     std::vector<int64_t> perm(pd->order.permtab.begin(), pd->order.permtab.end());
@@ -1682,10 +1692,8 @@ static int run_factor(pastix_data_t *pd, bool overlap) {
     PdlScope pdl_scope(two && sizeof(T) == 4);
     if (sizeof(T) == 4 || d.i8_on)
         CUDA_TRY(cudaMemsetAsync(d.queues.p, 0, 3 * pd->levels.size() * sizeof(int), st));
-    if (sizeof(T) == 8 && F == pgpu::FACT_GETRF && d.i8_on) {
+    if (sizeof(T) == 8 && F == pgpu::FACT_GETRF && d.i8_on)
         CUDA_TRY(cudaMemsetAsync(d.i8_flag.p, 0, d.i8_flag.n * sizeof(int), st));
-        CUDA_TRY(cudaMemsetAsync(d.i8_bal.p, 0, d.i8_bal.n * sizeof(unsigned long long), st));
-    }
     if (two) {
         CUDA_TRY(cudaEventRecord(d.ev_chain[0], st));
         CUDA_TRY(cudaStreamWaitEvent(d.side, d.ev_chain[0], 0));
@@ -1777,7 +1785,8 @@ static int run_factor(pastix_data_t *pd, bool overlap) {
                 int *lflag = d.queues.p + 3 * l + 1;  // LU: the level has flagged sources
                 launch_cls(pd, PC_SPLIT, nsl, [&] {
                     pgpu::launch_split_i8<F>(ds, d.i8_slabs.p + lv.isl0, nsl, L, U, d.i8_off.p, d.i8_img0.p, d.i8_img1.p,
-                                             d.i8_sc0.p, d.i8_sc1.p, d.i8_bal.p, d.i8_flag.p, lflag, d.counters.p + 2, st);
+                                             d.i8_sc0.p, d.i8_sc1.p, d.csr_val.p, d.csr_diag.p, d.i8_flag.p, lflag,
+                                             d.counters.p + 2, st);
                 });
                 const int nnear = (two ? lv.upin : lv.upi1) - lv.upi0;
                 launch_cls(pd, PC_UPDATE_BIG, nnear, [&] {
@@ -1958,13 +1967,13 @@ extern "C" int pastix_subtask_bcsc2ctab(pastix_data_t *pd) {
     } else if (i8_want) {
         const size_t nr = pd->solver.rowidx.size(), n = (size_t)pd->n;
         const bool two = fk != pgpu::FACT_POTRF, lu = fk == pgpu::FACT_GETRF;
-        const size_t need = (two ? 2 : 1) * (i8_bytes + 8 * nr) + (lu ? 16 * n + 4 * (size_t)pd->solver.cblknbr : 0);
+        const size_t need = (two ? 2 : 1) * (i8_bytes + 8 * nr) + (lu ? 4 * (size_t)pd->solver.cblknbr : 0);
         size_t fr = 0, tot = 0;
         CUDA_TRY(cudaMemGetInfo(&fr, &tot));
         d.i8_on = fr >= need + I8_RESERVE + 64 * 8 * n && d.i8_img0.alloc(i8_bytes) == cudaSuccess &&
                   d.i8_sc0.alloc(nr) == cudaSuccess &&
                   (!two || (d.i8_img1.alloc(i8_bytes) == cudaSuccess && d.i8_sc1.alloc(nr) == cudaSuccess)) &&
-                  (!lu || (d.i8_flag.alloc(pd->solver.cblknbr) == cudaSuccess && d.i8_bal.alloc(2 * n) == cudaSuccess));
+                  (!lu || d.i8_flag.alloc(pd->solver.cblknbr) == cudaSuccess);
         if (!d.i8_on) {
             (void)cudaGetLastError();
             d.release_images();
@@ -2025,7 +2034,7 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
         } else {
             const std::vector<uintptr_t> key{1, (uintptr_t)fk, (uintptr_t)d.Lc.p, (uintptr_t)d.Uc.p, (uintptr_t)d.dinv.p,
                                              (uintptr_t)d.i8_img0.p, (uintptr_t)d.i8_img1.p, (uintptr_t)d.i8_sc0.p,
-                                             (uintptr_t)d.i8_sc1.p, (uintptr_t)d.i8_flag.p, (uintptr_t)d.i8_bal.p};
+                                             (uintptr_t)d.i8_sc1.p, (uintptr_t)d.i8_flag.p};
             rc = run_graphed(pd, key, run);
         }
     }

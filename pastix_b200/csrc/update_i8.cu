@@ -24,22 +24,20 @@
 // Rounding relative to the row's largest entry asks for columns of like size:
 // the rows of a Cholesky factor are bounded by the diagonal of A, those of L in
 // LDL^T and LU are not (a small pivot makes a large column).  There column c is
-// scaled by a power of two h_c, exactly: (L h)(L D / h)^T and (L h)(U / h).
-// LDL^T: h_c = 2^(half the exponent of the pivot), the balance that Cholesky has.
-// LU: the pivot does not tell how a scaling of the matrix splits between L and U
-// (scaled rows change L alone by column, scaled columns U alone), so h_c comes
-// from the panels: log2 of their entries is taken as row part + column part, both
-// by least squares (the model of Curtis and Reid, J. Inst. Maths Applics 10,
-// 1972, one sweep, exact for a panel without zeros), and h_c is half of the column
-// part of U less that of L.  Scaling rows or columns of A by powers of two then
-// leaves the digits as they are.  A balance need not exist, so k_split_i8 also
-// checks that every row of L meets its row of U^T: sum_c |l_c u_c| is at least
-// 2^-8 of the product of their largest entries.  That sum is what bounds the FP64
-// rounding of the diagonal entry, about 2^-50.5 of it for 128 columns; 2^-60 a b is
-// then at most 2^-50 of it (LL^T and LDL^T: 2^-58, without a check).  A source with a
-// row that fails, with a row of one factor only, or beyond the range of the scales,
-// is flagged and updated by DMMA instead (launch_update_flagged).  Convection-
-// diffusion on 16 x 15 x 17 to 45 x 38 x 41 points: the smallest ratio is 2^-3.3.
+// scaled by h_c = 2^(half the exponent of the pivot), exactly: (L h)(L D / h)^T
+// and (L h)(U / h), the balance that Cholesky has.  LDL^T keeps the bound with
+// f_i = sum_c |l_ic d_c l_ic|, which bounds its FP64 rounding at (i, i), in place of
+// A_ii: a^2 <= 16 f_i by construction.  In LU that holds only while L and U share
+// their scaling; a matrix with rows or columns scaled on one side does not.  So
+// k_split_i8 checks every row: the squares of its largest entries in L h and U / h
+// are at most I8_OVER = 64 times max(|A_ii|, f_i), f_i = sum_c |l_ic u_ci|.  The error at
+// (i, j) is then at most 2^-52 sqrt(g_i g_j) (g: that maximum).  A source with a row that fails (or with one beyond the range of the
+// scales, or not finite) is flagged and updated by DMMA instead
+// (launch_update_flagged), whose FP64 products such scalings leave unchanged.
+// Flagged, of the 132 sources of a 32^3 convection-diffusion: none, nor with 30 to 80 %
+// of the off-diagonal entries dropped at random or scaled over 8 decades each; 6 with
+// one direction's cut to 10^-8; 129 with every other row and column in other units
+// (2^40, 2^30).
 //
 // Why: the FP64 tensor cores (DMMA) multiply 64 x 2 flops per clock and SM, the
 // 8-bit ones 8192 x 2; 36 digit products per FP64 product are 3.6 times fewer
@@ -71,7 +69,7 @@ constexpr int I8_BN = 128;
 constexpr int I8_TQ = 4;                   // tile-index ring
 constexpr int FAR_TILES_I8 = 6;            // tiles of a CTA of the far updates, about 80 us: 60^3 Laplacian,
                                            // factorization 15.7 -> 13.9 ms against one stream (far_grid)
-constexpr double I8_MEET = 0x1p-8;         // LU: least ratio of sum_c |l_c u_c| to max_c |l_c| max_c |u_c|
+constexpr double I8_OVER = 64.0;           // LU: bound on the square of a row's largest entry over its diagonal's scale
 constexpr int I8_MAX_K = 512;              // widest source: the sums i + j >= 4 stay within 2^50
 
 __host__ __device__ inline int i8_nkb(int nc) { return (nc + I8_KB - 1) / I8_KB; }
@@ -81,70 +79,6 @@ int far_grid(int count, int quota);  // factor.cu
 
 long long i8_image_bytes(int nc, int st) { return (long long)I8_S * i8_nkb(nc) * i8_ng(st) * I8_GROUP; }
 int i8_max_k() { return I8_MAX_K; }
-
-// ---------------------------------------------------------------------------
-// LU: the column parts of log2 |entry| in the rows below the diagonal block.
-// blockIdx.z: L or U^T; a lane holds a row, warps share the columns.  Pass one
-// finds each row's mean exponent, pass two (the slab is in L1 / L2 by then) adds
-// the exponents less their row's mean to bal, one word per column and side: the
-// sum in 16ths above 24 bits that count the nonzero entries.  Bound by HBM, the
-// panels of the sources read once more.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_balance_i8(DevStruct s, const SplitSlab *__restrict__ slabs, const double *L,
-                                                    const double *U, unsigned long long *bal) {
-    __shared__ int rsum[8][32], rcnt[8][32];
-    const SplitSlab sl = slabs[blockIdx.x];
-    const int k = sl.cblk;
-    const int nc = s.cb_lcol[k] - s.cb_fcol[k] + 1;
-    const int st = s.cb_stride[k];
-    const int r0 = sl.r0 + 32 * blockIdx.y;
-    if (r0 >= st || r0 + 32 <= nc) return;  // whole CTA
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pr = r0 + lane;
-    const bool in = pr >= nc && pr < st;
-    const double *A = (blockIdx.z ? U : L) + s.cb_coef[k] + pr;
-    auto expo = [&](int c, int (&e)[8]) {  // of columns c, c + 8, ..; 0: zero, subnormal or not finite
-        double v[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = (in && c + 8 * j < nc) ? A[(size_t)(c + 8 * j) * st] : 0.0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            e[j] = (__double2hiint(v[j]) >> 20) & 0x7ff;
-            if (e[j] == 0x7ff) e[j] = 0;
-        }
-    };
-    int sum = 0, cnt = 0;
-    for (int c = warp; c < nc; c += 64) {
-        int e[8];
-        expo(c, e);
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            sum += e[j];
-            cnt += e[j] != 0;
-        }
-    }
-    rsum[warp][lane] = sum;
-    rcnt[warp][lane] = cnt;
-    __syncthreads();
-    sum = cnt = 0;
-#pragma unroll
-    for (int w = 0; w < 8; w++) {
-        sum += rsum[w][lane];
-        cnt += rcnt[w][lane];
-    }
-    const int mean = cnt ? 16 * sum / cnt : 0;
-    unsigned long long *dst = bal + 2 * (size_t)s.cb_fcol[k] + blockIdx.z;
-    for (int c = warp; c < nc; c += 64) {
-        int e[8];
-        expo(c, e);
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int x = __reduce_add_sync(0xffffffffu, e[j] ? 16 * e[j] - mean : 0);
-            const int num = __popc(__ballot_sync(0xffffffffu, e[j] != 0));
-            if (lane == 0 && num)
-                atomicAdd(dst + 2 * (size_t)(c + 8 * j), (unsigned long long)(x * (1LL << 24) + num));
-        }
-    }
-}
 
 // ---------------------------------------------------------------------------
 // Digits of 32-row slabs (blockIdx.y) of 128-row panel slabs, of both operands
@@ -160,8 +94,9 @@ template <int FACT>
 __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *__restrict__ slabs, const double *L,
                                                   const double *U, const int64_t *__restrict__ i8_off,
                                                   unsigned char *img0, unsigned char *img1, double *__restrict__ sc0,
-                                                  double *__restrict__ sc1, const unsigned long long *__restrict__ bal,
-                                                  int *flag, int *level_flag, int *flagged) {
+                                                  double *__restrict__ sc1, const double *__restrict__ val,
+                                                  const int *__restrict__ diag_pos, int *flag, int *level_flag,
+                                                  int *flagged) {
     constexpr int SIDES = FACT == FACT_POTRF ? 1 : 2;
     constexpr bool LU = FACT == FACT_GETRF;
     __shared__ double red[SIDES][8][32], fsum[LU ? 8 : 1][32];
@@ -191,26 +126,13 @@ __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *
             }
         }
     };
-    if (FACT == FACT_SYTRF) {
+    if (FACT != FACT_POTRF) {
         for (int c = threadIdx.x; c < nc; c += 256) {
             const double d = L[s.cb_coef[k] + c + (size_t)c * st];
             const int e = (__double2hiint(d) >> 20) & 0x7ff;
             const int h = (e == 0 || e == 0x7ff) ? 0 : (e - 1023) / 2;  // zero and non-finite pivots: none
             colf[0][c] = i8_pow2(h);
-            colf[SIDES - 1][c] = d * i8_pow2(-h);
-        }
-        __syncthreads();
-    }
-    if (LU) {
-        for (int c = threadIdx.x; c < nc; c += 256) {
-            const long long bl = (long long)bal[2 * (size_t)(s.cb_fcol[k] + c)];
-            const long long bu = (long long)bal[2 * (size_t)(s.cb_fcol[k] + c) + 1];
-            const int nl = (int)(bl & 0xffffff), nu = (int)(bu & 0xffffff);
-            int h = 0;  // a column without entries on one side: none
-            if (nl && nu) h = __float2int_rn(((float)(bu >> 24) / (float)nu - (float)(bl >> 24) / (float)nl) * 0x1p-5f);
-            h = max(-1000, min(1000, h));
-            colf[0][c] = i8_pow2(h);
-            colf[SIDES - 1][c] = i8_pow2(-h);
+            colf[SIDES - 1][c] = LU ? i8_pow2(-h) : d * i8_pow2(-h);
         }
         __syncthreads();
     }
@@ -249,12 +171,12 @@ __global__ void __launch_bounds__(256) k_split_i8(DevStruct s, const SplitSlab *
     if (LU && warp == 0) {
         // rows that the integer products cannot take: see the head of this file.  A
         // scaled entry that left the range of FP64 is among them (bad), and so is a
-        // source with a non-finite entry, which DMMA carries on.
-        const double ab = m[0] * m[SIDES - 1];
+        // non-finite one, which DMMA carries on.
         const bool off = pr >= nc && pr < st;
-        const bool fails = bad || (m[0] > 0.0) != (m[SIDES - 1] > 0.0) ||
-                           (m[0] > 0.0 && !(ab >= 0x1p-1000 && f <= 0x1p1000 && f >= I8_MEET * ab &&
-                                            m[0] >= 0x1p-950 && m[SIDES - 1] >= 0x1p-950));
+        const int dp = off ? diag_pos[s.rowidx[s.cb_rowidx[k] + pr]] : -1;
+        const double aii = dp >= 0 ? fabs(val[dp]) : 0.0, g = I8_OVER * (aii > f ? aii : f);
+        auto fits = [&](double x) { return x == 0.0 || (x >= 0x1p-500 && x <= 0x1p500 && x * x <= g); };
+        const bool fails = bad || !fits(m[0]) || !fits(m[SIDES - 1]);
         if (__any_sync(0xffffffffu, off && fails) && lane == 0) {
             *level_flag = 1;
             if (atomicExch(flag + k, 1) == 0) atomicAdd(flagged, 1);
@@ -624,11 +546,11 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
 template <int FACT>
 void launch_split_i8(const DevStruct &s, const SplitSlab *slabs, int count, const double *L, const double *U,
                      const int64_t *i8_off, unsigned char *img0, unsigned char *img1, double *sc0, double *sc1,
-                     unsigned long long *bal, int *flag, int *level_flag, int *flagged, cudaStream_t st) {
+                     const double *val, const int *diag_pos, int *flag, int *level_flag, int *flagged,
+                     cudaStream_t st) {
     if (count <= 0) return;
-    if (FACT == FACT_GETRF) k_balance_i8<<<dim3(count, 4, 2), 256, 0, st>>>(s, slabs, L, U, bal);
-    k_split_i8<FACT><<<dim3(count, 4), 256, 0, st>>>(s, slabs, L, U, i8_off, img0, img1, sc0, sc1, bal, flag, level_flag,
-                                                     flagged);
+    k_split_i8<FACT><<<dim3(count, 4), 256, 0, st>>>(s, slabs, L, U, i8_off, img0, img1, sc0, sc1, val, diag_pos, flag,
+                                                     level_flag, flagged);
 }
 template <int FACT>
 void launch_update_i8(const DevStruct &s, const UpdTile *tiles, int count, double *L, double *U,
@@ -649,7 +571,7 @@ cudaError_t set_i8_attrs() {
 #define PGPU_INST_I8(F)                                                                                               \
     template void launch_split_i8<F>(const DevStruct &, const SplitSlab *, int, const double *, const double *,       \
                                      const int64_t *, unsigned char *, unsigned char *, double *, double *,           \
-                                     unsigned long long *, int *, int *, int *, cudaStream_t);                        \
+                                     const double *, const int *, int *, int *, int *, cudaStream_t);                 \
     template void launch_update_i8<F>(const DevStruct &, const UpdTile *, int, double *, double *,                    \
                                       const unsigned char *, const unsigned char *, const double *, const double *,   \
                                       const int64_t *, const int *, const int *, int *, int *, bool, cudaStream_t);

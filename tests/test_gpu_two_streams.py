@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
+import scipy.sparse as sps
 import torch
 
 from conftest import analyse
@@ -36,11 +37,8 @@ def test_two_streams_give_the_factors_of_one(lib, fact, uneven):
     grid = (36, 36, 36) if fact == "GETRF" else (48, 48, 48)
     A = gen.convdiff27(*grid) if fact == "GETRF" else gen.laplacian7(*grid)
     rng = np.random.default_rng(5)
-    if uneven:  # rows of L and U large in different columns, in a part of the domain
-        C = A.tocoo()
-        weak = (C.row != C.col) & (C.row < A.shape[0] // 8) & (rng.random(C.nnz) < 0.5)
-        C.data[weak] *= 1e-9
-        A = C.tocsc()
+    if uneven:  # rows of a part of the domain in other units: some sources are left to DMMA
+        A = (sps.diags(np.where(np.arange(A.shape[0]) < A.shape[0] // 8, 2.0 ** 20, 1.0)) @ A).tocsc()
     pd, S, info = analyse(A, grid, fact)
     assert info["thflops"] >= 2e10
     keep = _mask_compare(fact, info)

@@ -80,33 +80,76 @@ def test_scaled_rows(lib, fact, decades):
     px.finalize(pd)
 
 
-@pytest.mark.parametrize("decades", [0, 8, 14, 40, 200])
-@pytest.mark.parametrize("rows,cols", [(1, 0), (0, 1), (1, 1), (1, 2)])
-def test_lu_of_scaled_rows_and_columns(lib, decades, rows, cols):
+def _lu_error(M, grid, A, xt, l, r, integer=True, **kw):
+    """Relative error in the unscaled unknowns of M = 2^l A 2^r, and the sources handed back to FP64 arithmetic."""
+    pd, S, info = analyse(M, grid, "GETRF", **kw)
+    pd.dparm[px.dparm.epsilon_magn_ctrl] = -1e-300
+    px.integer_updates(pd, integer)
+    px.task_numfact(pd, S)
+    assert int(pd.iparm[px.iparm.static_pivoting]) == 0
+    b = np.ldexp(A @ xt, l)
+    px.task_solve(pd, S, b)
+    used, flagged = px.get_update_path(pd)
+    assert used == integer
+    nc, st = info["cb_lcol"] - info["cb_fcol"] + 1, info["cb_stride"]
+    sources = int(((nc >= 32) & (nc <= 512) & (nc * st > 4096) & (st > nc)).sum())
+    px.finalize(pd)
+    return np.linalg.norm(np.ldexp(b, r) - xt) / np.linalg.norm(xt), flagged / sources
+
+
+@pytest.mark.parametrize("decades", [8, 14, 40, 200])
+@pytest.mark.parametrize("kind", ["rows", "columns", "rows and columns", "both alike", "rows of one half"])
+def test_lu_of_scaled_rows_and_columns(lib, decades, kind):
     """D1 A D2 with powers of two drawn per row and column: FP64 elimination without pivoting does the same
     arithmetic for every such scaling, so the error in the unscaled unknowns is that of A itself (twice that is
     allowed for the order of the scattered sums)."""
     A, grid = gen.convdiff27(16, 15, 17), (16, 15, 17)
     n = A.shape[0]
     rng = np.random.default_rng(7)
-    draw = [rng.integers(-int(1.66 * decades), int(1.66 * decades) + 1, n) for _ in range(2)]
-    l = rows * draw[0] // (1 + (rows == cols))
-    r = draw[0] // 2 if rows == cols else (cols > 0) * draw[cols - 1]
+    l, r = (rng.integers(-int(1.66 * decades), int(1.66 * decades) + 1, n) for _ in range(2))
+    if kind == "rows":
+        r = 0 * r
+    elif kind == "columns":
+        l = 0 * l
+    elif kind == "both alike":
+        l = r = l // 2
+    elif kind == "rows of one half":
+        l, r = np.where(np.arange(n) < n // 2, int(3.3 * decades), 0), 0 * r
     xt = gen.rhs_uniform(n, 1, 3)[:, 0]
-    err = []
-    for lq, rq in ((0 * l, 0 * r), (l, r)):
-        M = (sps.diags(np.ldexp(1.0, lq)) @ A @ sps.diags(np.ldexp(1.0, rq))).tocsc()
-        pd, S, info = analyse(M, grid, "GETRF")
-        pd.dparm[px.dparm.epsilon_magn_ctrl] = -1e-300
-        px.task_numfact(pd, S)
-        assert int(pd.iparm[px.iparm.static_pivoting]) == 0
-        b = np.ldexp(A @ xt, lq)
-        px.task_solve(pd, S, b)
-        err.append(np.linalg.norm(np.ldexp(b, rq) - xt) / np.linalg.norm(xt))
-        used, flagged = px.get_update_path(pd)
-        assert used and (flagged == 0 or decades > 14)
-        px.finalize(pd)
-    assert err[1] < 2 * err[0], err
+    ref, flagged = _lu_error(A, grid, A, xt, 0 * l, 0 * r)
+    assert flagged == 0
+    M = (sps.diags(np.ldexp(1.0, l)) @ A @ sps.diags(np.ldexp(1.0, r))).tocsc()
+    err, flagged = _lu_error(M, grid, A, xt, l, r)
+    assert err < 2 * ref, (err, ref)
+    assert (flagged > 0) == (kind != "both alike")
+    assert kind != "rows of one half" or flagged < 1
+
+
+@pytest.mark.parametrize("kind", ["dropped", "most dropped", "one direction", "lower", "uneven"])
+def test_lu_of_unsymmetric_matrices(lib, kind):
+    """Unsymmetric patterns, weak couplings in one direction, entries of very different sizes: the slices keep them,
+    with the error of FP64 arithmetic (twice that for the order of the scattered sums)."""
+    A, grid = gen.convdiff27(24, 23, 25), (24, 23, 25)
+    n = A.shape[0]
+    rng = np.random.default_rng(11)
+    C = A.tocoo()
+    off = C.row != C.col
+    if kind == "dropped":
+        C.data[off & (rng.random(C.nnz) < 0.3)] = 0.0
+    elif kind == "most dropped":
+        C.data[off & (rng.random(C.nnz) < 0.8)] = 0.0
+    elif kind == "one direction":
+        C.data[C.row < C.col] *= 1e-8
+    elif kind == "lower":
+        C.data[C.row < C.col] = 0.0
+    else:
+        C.data[off] *= 10.0 ** rng.uniform(-8, 0, int(off.sum()))
+    A = C.tocsc()
+    xt = gen.rhs_uniform(n, 1, 3)[:, 0]
+    z = np.zeros(n, dtype=int)
+    ref, _ = _lu_error(A, grid, A, xt, z, z, integer=False, min_bs=64, max_bs=128)
+    err, flagged = _lu_error(A, grid, A, xt, z, z, min_bs=64, max_bs=128)
+    assert err < 2 * ref and flagged == 0, (err, ref, flagged)
 
 
 def _dense_chain(A, fact, width):
@@ -183,31 +226,6 @@ def test_updates_lose_nothing_against_fp64(lib, fact, width):
         e64 = np.triu((_lu(A, width) - ref).astype(float), 1)
         err = np.linalg.norm(Ut - np.triu(ref, 1).T.astype(float))
         assert err < 1.5 * np.linalg.norm(e64)
-    px.finalize(pd)
-
-
-@pytest.mark.parametrize("width", [32, 64, 100])
-def test_lu_rows_of_one_factor_only(lib, width):
-    """Rows that have entries in L but none in U, or large ones in different columns: those sources go to DMMA,
-    the others stay; the error is that of FP64."""
-    n = 520
-    rng = np.random.default_rng(3)
-    A = np.exp(-np.abs(np.subtract.outer(np.arange(n), np.arange(n))) / 20.0) * rng.uniform(0.5, 1.5, (n, n))
-    A[np.arange(n), np.arange(n)] = 40.0
-    A[300:320, :120] = 0.0   # no L part in the first panels
-    A[400:420, :64] *= 1e-9  # L and U of these rows large in different columns
-    A[:64, 400:420] *= 1e-9
-    A[410, 3] = A[3 + 20, 410] = 1.0
-    ref = _lu(A.astype(np.longdouble), 0)
-    e64 = (_lu(A, width) - ref).astype(float)
-    pd, S, info = _dense_chain(A, "GETRF", width)
-    px.task_numfact(pd, S)
-    used, flagged = px.get_update_path(pd)
-    assert used and 0 < flagged < int(info["cblknbr"])
-    Lg, Ug = px.get_coeftab(pd, with_u=True)
-    for F, tri, base in ((_dense_factor(info, Lg), np.tril(ref, -1), np.tril(e64, -1)),
-                         (_dense_factor(info, Ug), np.triu(ref, 1).T, np.triu(e64, 1))):
-        assert np.linalg.norm((np.tril(F, -1) - tri).astype(float)) < 1.5 * np.linalg.norm(base)
     px.finalize(pd)
 
 
