@@ -2065,7 +2065,10 @@ extern "C" int pastix_subtask_sopalin(pastix_data_t *pd) {
 static int factor_values(pastix_data_t *pd) {
     int rc = pastix_subtask_bcsc2ctab(pd);
     if (!rc) rc = pastix_subtask_sopalin(pd);
-    if (rc) (void)fetch_norm(pd);
+    if (rc) {
+        if (pd->dev.side) (void)cudaStreamSynchronize(pd->dev.side);  // far updates that were launched before the failure
+        (void)fetch_norm(pd);
+    }
     return rc;
 }
 
